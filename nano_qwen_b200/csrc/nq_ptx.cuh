@@ -2,10 +2,10 @@
 // (cp.async.bulk.tensor, never with cluster multicast), tcgen05 (TMEM
 // allocation, UMMA issue/commit, TMEM loads) and bounded waits.
 //
-// Every wait on an mbarrier goes through mbar_wait(), which gives up after a
-// wall-clock limit, raises a CTA-wide abort flag and records where it gave up;
-// callers leave their loop and fall through to the common teardown, so a
-// kernel never spins forever and never traps.
+// Every wait on an mbarrier goes through WaitCtl::wait(), which gives up after
+// a wall-clock limit, raises a CTA-wide abort flag and remembers where it gave
+// up; the caller runs on to the common teardown, so a kernel never spins
+// forever and never traps.
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -64,100 +64,80 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Non-blocking probe of the same condition (never suspends the thread).
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool mbar_try_wait_hint(uint64_t* bar, uint32_t parity, uint32_t ns) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity), "r"(ns)
-      : "memory");
-  return ok != 0;
+// One lane of a converged warp.  A loop that issues tcgen05 / TMA instructions belongs under `if (elect_one())` with the
+// warp index taken through __shfl_sync: the compiler then knows that a single thread runs it and keeps descriptors and
+// barrier addresses in uniform registers.  Under `if (lane == 0)` the same four UMMAs and two commits of a K-tile cost
+// the issuing thread 274 cycles instead of 161 (128 x 32 x 32 UMMAs, measured in isolation).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
 }
 
-// Shared by all roles of a CTA: raised once, never cleared during the launch.
-struct AbortCtl {
-  volatile int* flag;       // in shared memory
-  DeviceStatus* status;     // mapped host memory (may be null)
-  uint64_t limit_ns;        // wall-clock limit for one wait
-  uint32_t wait_mode;       // 0 try_wait, 1 test_wait spin, >1 try_wait with that suspend-time hint (ns)
-};
-
-static __device__ __noinline__ void report_timeout(const AbortCtl& ac, int where, int aux) {
-  *ac.flag = 1;
-  if (ac.status != nullptr) {
-    if (atomicCAS(&ac.status->code, 0, kErrDeviceTimeout) == 0) {
-      ac.status->where = where;
-      ac.status->block = static_cast<int>(blockIdx.x);
-      ac.status->aux = aux;
+static __device__ __noinline__ void report_timeout(DeviceStatus* status, int where, int aux) {
+  if (status != nullptr) {
+    if (atomicCAS(&status->code, 0, kErrDeviceTimeout) == 0) {
+      status->where = where;
+      status->block = static_cast<int>(blockIdx.x);
+      status->aux = aux;
       __threadfence_system();
     }
   }
 }
 
-// Waits for the phase with the given parity.  Returns false when the CTA is
-// aborting (this wait or another one ran out of time).
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const AbortCtl& ac, int where, int aux) {
-  if (mbar_try_wait(bar, parity)) return true;
-  // The limit is checked against the SM cycle counter (cheap to read; ~2 GHz, so
-  // 2 cycles per nanosecond is a generous conversion of the wall-clock limit).
-  const long long t0 = clock64();
-  const long long limit_cycles = static_cast<long long>(ac.limit_ns) * 2;
-  for (uint32_t spin = 1;; ++spin) {
-    if (ac.wait_mode == 1) { if (mbar_test_wait(bar, parity)) return true; }
-    else if (ac.wait_mode > 1) { if (mbar_try_wait_hint(bar, parity, ac.wait_mode)) return true; }
-    else if (mbar_try_wait(bar, parity)) return true;
-    if ((spin & 255u) == 0u) {
-      if (*ac.flag) return false;
-      if (clock64() - t0 > limit_cycles) {
-        report_timeout(ac, where, aux);
-        return false;
-      }
-    }
-  }
-}
+// Bounded waits of one role of a CTA.
+//
+// wait() returns when the phase with the given parity is complete, or when it has waited for the limit, or when another
+// role of the CTA has given up (the abort flag in shared memory).  It never branches in the calling code: after a
+// give-up `limit` is 0 and every further wait of the thread falls through at once, so the role's loop runs to its end
+// on whatever the buffers hold - its UMMAs, loads and stores stay inside the same buffers - and the kernel ends by its
+// common teardown.  Only a TMA producer has to look at gave_up() (it must not leave copies in flight behind).
+// All control flow is inside the asm statement on purpose: a C++ loop with a give-up branch around the same
+// instructions costs the UMMA issuing thread about 220 cycles per K-tile (128 x 128 x 128: 498 cycles instead of 277),
+// more than the tensor core's two queued UMMAs can hide.
+// The limit is checked against the SM cycle counter (cheap to read; 2 cycles per nanosecond is a generous conversion).
+struct WaitCtl {
+  uint64_t limit;      // cycles; 0 after a give-up
+  uint32_t flag;       // shared-memory address of the CTA's abort flag
+  uint32_t site;       // 0, or wait site | aux << 8 of this thread's first expired wait
 
-// Same bounded wait with cluster-scope acquire: the barrier is completed by another CTA of the cluster
-// (remote arrivals, or copies issued by the peer).
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, const AbortCtl& ac, int where, int aux) {
-  if (mbar_try_wait_cluster(bar, parity)) return true;
-  const long long t0 = clock64();
-  const long long limit_cycles = static_cast<long long>(ac.limit_ns) * 2;
-  for (uint32_t spin = 1;; ++spin) {
-    if (mbar_try_wait_cluster(bar, parity)) return true;
-    if ((spin & 255u) == 0u) {
-      if (*ac.flag) return false;
-      if (clock64() - t0 > limit_cycles) {
-        report_timeout(ac, where, aux);
-        return false;
-      }
-    }
+  __device__ __forceinline__ WaitCtl(int* abort_flag, uint64_t limit_ns) : limit(limit_ns * 2), flag(smem_u32(abort_flag)), site(0) {}
+
+  __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity, uint32_t where, uint32_t aux) {
+    asm volatile(
+        "{\n\t.reg .pred P;\n\t.reg .u64 t0, t1;\n\t.reg .u32 f;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P, [%2], %3;\n\t"
+        "@P bra DONE;\n\t"
+        "mov.u64 t0, %%clock64;\n\t"
+        "AGAIN:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P, [%2], %3;\n\t"
+        "@P bra DONE;\n\t"
+        "ld.volatile.shared.u32 f, [%4];\n\t"
+        "setp.ne.u32 P, f, 0;\n\t"
+        "@P bra STOP;\n\t"
+        "mov.u64 t1, %%clock64;\n\t"
+        "sub.u64 t1, t1, t0;\n\t"
+        "setp.lt.u64 P, t1, %0;\n\t"
+        "@P bra AGAIN;\n\t"
+        "shl.b32 f, %6, 8;\n\t"
+        "or.b32 %1, f, %5;\n\t"
+        "mov.u32 f, 1;\n\t"
+        "st.volatile.shared.u32 [%4], f;\n\t"
+        "STOP:\n\t"
+        "mov.u64 %0, 0;\n\t"
+        "DONE:\n\t}"
+        : "+l"(limit), "+r"(site)
+        : "r"(bar), "r"(parity), "r"(flag), "r"(where), "r"(aux)
+        : "memory");
   }
-}
+  __device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity, uint32_t where, uint32_t aux) {
+    wait(smem_u32(bar), parity, where, aux);
+  }
+  __device__ __forceinline__ bool gave_up() const { return limit == 0; }
+  __device__ __forceinline__ void report(DeviceStatus* status) const {
+    if (site != 0) report_timeout(status, static_cast<int>(site & 255u), static_cast<int>(site >> 8));
+  }
+};
 
 // ---------------------------------- TMA ------------------------------------ //
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
