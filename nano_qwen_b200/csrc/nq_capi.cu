@@ -101,18 +101,20 @@ int cached_encode(CUtensorMap* out, const TmapKey& k) {
   h ^= static_cast<uint64_t>(k.ld) * 0x27D4EB2F165667C5ull + static_cast<uint64_t>(k.box_rows * 4 + k.box_cols * 4096 + k.kind);
   TmapSlot& slot = t_tmap_cache[(h >> 32) % kTmapSlots];
   if (slot.valid && slot.key == k) { *out = slot.map; return NQ_OK; }
+  static constexpr CUtensorMapDataType kType[3] = {CU_TENSOR_MAP_DATA_TYPE_UINT8, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
+                                                   CU_TENSOR_MAP_DATA_TYPE_FLOAT32};
+  static constexpr const char* kName[3] = {"u8", "bf16", "f32"};
   const bool u8 = (k.kind == 0);
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(k.cols), static_cast<cuuint64_t>(k.rows)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(k.ld) * (u8 ? 1 : 2)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(k.ld) << k.kind};       // element sizes 1, 2, 4
   const cuuint32_t box[2] = {static_cast<cuuint32_t>(k.box_cols), static_cast<cuuint32_t>(k.box_rows)};
   const cuuint32_t elem[2] = {1u, 1u};
-  const CUresult r = g_encode(out, u8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
-                              const_cast<void*>(k.base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              u8 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+  const CUresult r = g_encode(out, kType[k.kind], 2, const_cast<void*>(k.base), dims, strides, box, elem,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, u8 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                               u8 ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_NONE,
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
-    snprintf(t_cuda_err, sizeof(t_cuda_err), "cuTensorMapEncodeTiled (%s) failed with CUresult %d", u8 ? "u8" : "bf16",
+    snprintf(t_cuda_err, sizeof(t_cuda_err), "cuTensorMapEncodeTiled (%s) failed with CUresult %d", kName[k.kind],
              static_cast<int>(r));
     return NQ_ERR_CUDA;
   }
@@ -130,6 +132,10 @@ int make_tmap_u8_2d(CUtensorMap* out, const void* base, int64_t rows, int64_t co
 int make_tmap_bf16_2d(CUtensorMap* out, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_rows,
                       int box_cols) {
   return cached_encode(out, TmapKey{base, rows, cols, ld, box_rows, box_cols, 1});
+}
+
+int make_tmap_f32_2d(CUtensorMap* out, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_rows, int box_cols) {
+  return cached_encode(out, TmapKey{base, rows, cols, ld, box_rows, box_cols, 2});
 }
 
 namespace {
