@@ -20,7 +20,7 @@ struct DeviceStatus {
   int code;        // 0 = OK, else an NQ_ERR_* value written by the first failing CTA
   int where;       // site id of the wait that expired
   int block;       // blockIdx.x of the reporter
-  int aux;         // site-specific (stage / K-tile index)
+  int aux;         // site-specific (GEMM: blockIdx.y; reductions: the peer)
 };
 
 constexpr int kErrDeviceTimeout = -5;  // mirrors NQ_ERR_DEVICE_TIMEOUT in include/nq_fp8.h
@@ -74,12 +74,12 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 
-static __device__ __noinline__ void report_timeout(DeviceStatus* status, int where, int aux) {
+static __device__ __noinline__ void report_timeout(DeviceStatus* status, int where) {
   if (status != nullptr) {
     if (atomicCAS(&status->code, 0, kErrDeviceTimeout) == 0) {
       status->where = where;
       status->block = static_cast<int>(blockIdx.x);
-      status->aux = aux;
+      status->aux = static_cast<int>(blockIdx.y);
       __threadfence_system();
     }
   }
@@ -97,13 +97,17 @@ static __device__ __noinline__ void report_timeout(DeviceStatus* status, int whe
 // more than the tensor core's two queued UMMAs can hide.
 // The limit is checked against the SM cycle counter (cheap to read; 2 cycles per nanosecond is a generous conversion).
 struct WaitCtl {
-  uint64_t limit;      // cycles; 0 after a give-up
+  uint32_t limit;      // units of 1024 cycles; 0 after a give-up
   uint32_t flag;       // shared-memory address of the CTA's abort flag
-  uint32_t site;       // 0, or wait site | aux << 8 of this thread's first expired wait
+  uint32_t site;       // wait site of this thread's first expired wait (0: none)
 
-  __device__ __forceinline__ WaitCtl(int* abort_flag, uint64_t limit_ns) : limit(limit_ns * 2), flag(smem_u32(abort_flag)), site(0) {}
+  __device__ __forceinline__ WaitCtl(int* abort_flag, uint64_t limit_ns) : flag(smem_u32(abort_flag)), site(0) {
+    const uint64_t units = (limit_ns >> 9) + 1;
+    limit = units < 0x7FFFFFFFull ? static_cast<uint32_t>(units) : 0x7FFFFFFFu;
+  }
 
-  __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity, uint32_t where, uint32_t aux) {
+  template <int SITE>
+  __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity) {
     asm volatile(
         "{\n\t.reg .pred P;\n\t.reg .u64 t0, t1;\n\t.reg .u32 f;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 P, [%2], %3;\n\t"
@@ -117,27 +121,44 @@ struct WaitCtl {
         "@P bra STOP;\n\t"
         "mov.u64 t1, %%clock64;\n\t"
         "sub.u64 t1, t1, t0;\n\t"
-        "setp.lt.u64 P, t1, %0;\n\t"
+        "shr.u64 t1, t1, 10;\n\t"
+        "cvt.u32.u64 f, t1;\n\t"
+        "setp.lt.u32 P, f, %0;\n\t"
         "@P bra AGAIN;\n\t"
-        "shl.b32 f, %6, 8;\n\t"
-        "or.b32 %1, f, %5;\n\t"
+        "mov.u32 %1, %5;\n\t"
         "mov.u32 f, 1;\n\t"
         "st.volatile.shared.u32 [%4], f;\n\t"
         "STOP:\n\t"
-        "mov.u64 %0, 0;\n\t"
+        "mov.u32 %0, 0;\n\t"
         "DONE:\n\t}"
-        : "+l"(limit), "+r"(site)
-        : "r"(bar), "r"(parity), "r"(flag), "r"(where), "r"(aux)
+        : "+r"(limit), "+r"(site)
+        : "r"(bar), "r"(parity), "r"(flag), "n"(SITE)
         : "memory");
   }
-  __device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity, uint32_t where, uint32_t aux) {
-    wait(smem_u32(bar), parity, where, aux);
-  }
+  template <int SITE>
+  __device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity) { wait<SITE>(smem_u32(bar), parity); }
   __device__ __forceinline__ bool gave_up() const { return limit == 0; }
   __device__ __forceinline__ void report(DeviceStatus* status) const {
-    if (site != 0) report_timeout(status, static_cast<int>(site & 255u), static_cast<int>(site >> 8));
+    if (site != 0) report_timeout(status, static_cast<int>(site));
   }
 };
+
+// A value that the compiler does not know to be the same in all lanes: address arithmetic on it stays in ordinary registers.
+// (The epilogue's few address updates per K-tile, done in the uniform datapath, took 270 instructions per K-tile and SM
+// and a chain of their latencies on every warp.)
+__device__ __forceinline__ uint32_t per_lane(uint32_t v) {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %1;" : "=r"(r) : "r"(v));
+  return r;
+}
+__device__ __forceinline__ float ld_shared_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ void mbar_arrive_at(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 
 // ---------------------------------- TMA ------------------------------------ //
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
