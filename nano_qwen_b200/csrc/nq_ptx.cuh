@@ -420,6 +420,14 @@ struct ExactDivider {
     const float2 r = __ffma2_rn(make_float2(-s, -s), q0, x);
     return __ffma2_rn(r, y2, q0);
   }
+  // The same quotients x / s from nx = -x.  The residual has the opposite sign, so an exact zero of it cannot turn a
+  // quotient of -0 into +0: the bytes equal those of the IEEE divide for negative zeros too.
+  __device__ __forceinline__ float2 fast2_negated(float2 nx) const {
+    const float2 ny2 = make_float2(-y, -y);
+    const float2 q0 = __fmul2_rn(nx, ny2);
+    const float2 r = __ffma2_rn(make_float2(s, s), q0, nx);
+    return __ffma2_rn(r, ny2, q0);
+  }
 };
 
 // |a| max |b| element-wise on packed bf16 pairs (exact: a maximum never rounds).

@@ -103,37 +103,50 @@ __global__ void __launch_bounds__(256) act_quant_kernel(const __nv_bfloat16* __r
 }
 
 // ------------------------------------------------------------------------- //
-// Weight quantiser.  One CTA of 256 threads per 128x128 block; thread t owns
-// row t/2, 64 consecutive elements (columns (t&1)*64 ...).  Offline work.
+// Weight quantiser.  One CTA of 256 threads per 128x128 block, 16 lanes per row, 8 consecutive elements per lane
+// and row, 16 rows at a time.
+// Bound by HBM (2 bytes in, 1 byte out per weight): the block is read once and stays in registers between the amax
+// and the division (32 per thread), a half-warp reads 256 and writes 128 consecutive bytes, and the quotient costs
+// three packed instructions per pair instead of two IEEE divisions.  Two matrices of 12288 x 4096, written straight
+// into the merged parameter: 53 us = 5.7 TB/s (two passes of 128-byte segments per thread, IEEE divisions and a copy
+// of the result into the parameter: 168 us).
+// VEC: 16-byte loads and 8-byte stores, possible when K and both row strides are multiples of 8 and the bases are
+// aligned; otherwise element by element.
 // ------------------------------------------------------------------------- //
-__global__ void __launch_bounds__(256) weight_quant_kernel(const __nv_bfloat16* __restrict__ w, int64_t N, int64_t K,
-                                                           int64_t ldw, uint8_t* __restrict__ wq, int64_t ld_wq,
-                                                           float* __restrict__ sw, int64_t ld_sw, int vec) {
+template <bool VEC>
+__global__ void __launch_bounds__(256, 4) weight_quant_kernel(const __nv_bfloat16* __restrict__ w, int64_t N, int64_t K,
+                                                              int64_t ldw, uint8_t* __restrict__ wq, int64_t ld_wq,
+                                                              float* __restrict__ sw, int64_t ld_sw) {
   __shared__ float warp_max[8];
   const int64_t bk = blockIdx.x, bn = blockIdx.y;
-  const int64_t n = bn * 128 + (threadIdx.x >> 1);
-  const int64_t k0 = bk * 128 + (threadIdx.x & 1) * 64;
-  float amax = 0.0f;
-  const bool row_ok = n < N;
-  if (row_ok) {
-    if (vec) {
-      const uint4* src = reinterpret_cast<const uint4*>(w + n * ldw + k0);
+  const int r0 = threadIdx.x >> 4;                       // this thread's rows of the block: r0 + 16 * i
+  const int rows = static_cast<int>(N - bn * 128 < 128 ? N - bn * 128 : 128);
+  const int64_t k0 = bk * 128 + (threadIdx.x & 15) * 8;
+  const __nv_bfloat16* src_row = w + (bn * 128 + r0) * ldw;
+  uint4 raw[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const uint4 a = __ldg(src + i);
-        const uint32_t u[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          amax = fmaxf(amax, fabsf(bf16_bits_to_float(u[j] & 0xFFFFu)));
-          amax = fmaxf(amax, fabsf(bf16_bits_to_float(u[j] >> 16)));
-        }
-      }
+  for (int i = 0; i < 8; ++i, src_row += 16 * ldw) {
+    raw[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (r0 + 16 * i >= rows || k0 >= K) continue;
+    if (VEC) {
+      raw[i] = __ldcs(reinterpret_cast<const uint4*>(src_row + k0));
     } else {
-      const unsigned short* src = reinterpret_cast<const unsigned short*>(w + n * ldw);
-      for (int i = 0; i < 64; ++i)
-        if (k0 + i < K) amax = fmaxf(amax, fabsf(bf16_bits_to_float(src[k0 + i])));
+      const unsigned short* src = reinterpret_cast<const unsigned short*>(src_row);
+      uint32_t u[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t lo = (k0 + 2 * j < K) ? src[k0 + 2 * j] : 0u;
+        const uint32_t hi = (k0 + 2 * j + 1 < K) ? src[k0 + 2 * j + 1] : 0u;
+        u[j] = lo | (hi << 16);
+      }
+      raw[i] = make_uint4(u[0], u[1], u[2], u[3]);
     }
   }
+  uint32_t m2 = 0u;                                      // packed pairs: a maximum of bf16 values is exact
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    m2 = bf16x2_absmax(m2, bf16x2_absmax(bf16x2_absmax(raw[i].x, raw[i].y), bf16x2_absmax(raw[i].z, raw[i].w)));
+  float amax = fmaxf(bf16_bits_to_float(m2 & 0xFFFFu), bf16_bits_to_float(m2 >> 16));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
   if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = amax;
@@ -143,34 +156,32 @@ __global__ void __launch_bounds__(256) weight_quant_kernel(const __nv_bfloat16* 
   for (int i = 1; i < 8; ++i) amax = fmaxf(amax, warp_max[i]);
   const float scale = __fdiv_rn(fmaxf(amax, 1e-10f), 448.0f);
   if (threadIdx.x == 0) sw[bn * ld_sw + bk] = scale;
-  if (!row_ok) return;
-  const unsigned short* src = reinterpret_cast<const unsigned short*>(w + n * ldw);
-  uint8_t* dst = wq + n * ld_wq;
-  if (vec) {
+  if (k0 >= K) return;
+  const ExactDivider div(scale);
+  uint8_t* dst = wq + (bn * 128 + r0) * ld_wq + k0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float v[16];
-      const uint4 a = __ldg(reinterpret_cast<const uint4*>(src + k0) + 2 * i);
-      const uint4 b = __ldg(reinterpret_cast<const uint4*>(src + k0) + 2 * i + 1);
-      const uint32_t u[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  for (int i = 0; i < 8; ++i, dst += 16 * ld_wq) {
+    if (r0 + 16 * i >= rows) break;
+    const uint32_t u[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+    float2 v[4];
+    if (!div.slow) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        v[2 * j] = __fdiv_rn(bf16_bits_to_float(u[j] & 0xFFFFu), scale);
-        v[2 * j + 1] = __fdiv_rn(bf16_bits_to_float(u[j] >> 16), scale);
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t neg = u[j] ^ 0x80008000u;
+        v[j] = div.fast2_negated(make_float2(__uint_as_float(neg << 16), __uint_as_float(neg & 0xFFFF0000u)));
       }
-      uint4 q;
-      q.x = pack4_e4m3(v[0], v[1], v[2], v[3]);
-      q.y = pack4_e4m3(v[4], v[5], v[6], v[7]);
-      q.z = pack4_e4m3(v[8], v[9], v[10], v[11]);
-      q.w = pack4_e4m3(v[12], v[13], v[14], v[15]);
-      *reinterpret_cast<uint4*>(dst + k0 + 16 * i) = q;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        v[j] = make_float2(__fdiv_rn(__uint_as_float(u[j] << 16), scale), __fdiv_rn(__uint_as_float(u[j] & 0xFFFF0000u), scale));
     }
-  } else {
-    for (int i = 0; i < 64; ++i) {
-      if (k0 + i < K) {
-        const float q = __fdiv_rn(bf16_bits_to_float(src[k0 + i]), scale);
-        dst[k0 + i] = static_cast<uint8_t>(__nv_cvt_float_to_fp8(q, __NV_SATFINITE, __NV_E4M3));
-      }
+    const uint2 q = make_uint2(pack4_e4m3(v[0].x, v[0].y, v[1].x, v[1].y), pack4_e4m3(v[2].x, v[2].y, v[3].x, v[3].y));
+    if (VEC) {
+      __stcs(reinterpret_cast<uint2*>(dst), q);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (k0 + j < K) dst[j] = static_cast<uint8_t>((j < 4 ? q.x : q.y) >> ((j & 3) * 8));
     }
   }
 }
@@ -210,11 +221,11 @@ int launch_act_quant(const void* x, int64_t M, int64_t K, int64_t ldx, void* xq,
 int launch_weight_quant(const void* w, int64_t N, int64_t K, int64_t ldw, void* wq, int64_t ld_wq, float* sw,
                         int64_t ld_sw, cudaStream_t stream) {
   if (N == 0 || K == 0) return NQ_OK;
-  const int vec = (K % 128 == 0) && (ldw % 8 == 0) && (ld_wq % 16 == 0) &&
-                  (reinterpret_cast<uintptr_t>(w) % 16 == 0) && (reinterpret_cast<uintptr_t>(wq) % 16 == 0);
-  dim3 grid(static_cast<unsigned>((K + 127) / 128), static_cast<unsigned>((N + 127) / 128));
-  weight_quant_kernel<<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(w), N, K, ldw,
-                                                static_cast<uint8_t*>(wq), ld_wq, sw, ld_sw, vec);
+  const bool vec = (K % 8 == 0) && (ldw % 8 == 0) && (ld_wq % 8 == 0) &&
+                   (reinterpret_cast<uintptr_t>(w) % 16 == 0) && (reinterpret_cast<uintptr_t>(wq) % 8 == 0);
+  const dim3 grid(static_cast<unsigned>((K + 127) / 128), static_cast<unsigned>((N + 127) / 128));
+  const auto kernel = vec ? weight_quant_kernel<true> : weight_quant_kernel<false>;
+  kernel<<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(w), N, K, ldw, static_cast<uint8_t*>(wq), ld_wq, sw, ld_sw);
   count_launch();
   return check_cuda(cudaGetLastError());
 }

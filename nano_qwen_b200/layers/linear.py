@@ -112,10 +112,14 @@ class LinearBase(nn.Module):
         if not self.weight.is_cuda:
             raise RuntimeError("quantising an unquantised checkpoint tensor needs the module on a CUDA device "
                                "(no CPU fallback); load pre-quantised float8 tensors instead")
-        wq, sw = ops.weight_quant(piece.to(device=self.weight.device, dtype=torch.bfloat16))
-        self.weight.data.narrow(dim, dst_offset, dst_size).copy_(wq)
+        w = piece.to(device=self.weight.device, dtype=torch.bfloat16)
+        rows = self.weight.data.narrow(dim, dst_offset, dst_size)
         off, size = self._to_units(self.weight_scale_inv, dim, dst_offset, dst_size)
-        self.weight_scale_inv.data.narrow(dim, off, size).copy_(sw)
+        scales = self.weight_scale_inv.data.narrow(dim, off, size)
+        if not ops.weight_quant_into(w, rows, scales):
+            wq, sw = ops.weight_quant(w)
+            rows.copy_(wq)
+            scales.copy_(sw)
 
     def _linear(self, x, bias: torch.Tensor | None) -> torch.Tensor:
         if isinstance(x, QuantizedActivation):       # a fused producer already quantised it: GEMM only

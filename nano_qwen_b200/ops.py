@@ -161,16 +161,44 @@ def weight_quant(w: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
     _require_cuda(w)
     if w.dtype != torch.bfloat16 or w.dim() != 2:
         raise TypeError("weight_quant expects a 2-D bfloat16 tensor")
-    w = w.contiguous()
     N, K = w.shape
     ld_wq = _round_up(max(K, 1), 16)
     wq_buf = torch.empty((N, ld_wq), dtype=FP8, device=w.device)
     sw = torch.empty(((N + GROUP - 1) // GROUP, (K + GROUP - 1) // GROUP), dtype=torch.float32, device=w.device)
-    if N > 0 and K > 0:
-        st = _cabi.lib().nq_weight_quant_e4m3_b128(w.data_ptr(), N, K, K, wq_buf.data_ptr(), ld_wq,
-                                                   sw.data_ptr(), sw.stride(0), _stream())
-        _cabi.check(st, "nq_weight_quant_e4m3_b128")
+    _launch_weight_quant(w, wq_buf[:, :K], sw)
     return wq_buf[:, :K], sw
+
+
+def _launch_weight_quant(w: torch.Tensor, wq: torch.Tensor, sw: torch.Tensor) -> None:
+    """``wq`` and ``sw`` have unit stride along their second dimension; ``w`` is copied unless its rows can be read in place."""
+    N, K = w.shape
+    if N == 0 or K == 0:
+        return
+    if (K > 1 and w.stride(1) != 1) or (N > 1 and w.stride(0) < K):
+        w = w.contiguous()
+    st = _cabi.lib().nq_weight_quant_e4m3_b128(
+        w.data_ptr(), N, K, w.stride(0) if N > 1 else K, wq.data_ptr(), wq.stride(0) if N > 1 else K,
+        sw.data_ptr(), sw.stride(0) if sw.shape[0] > 1 else sw.shape[1], _stream())
+    _cabi.check(st, "nq_weight_quant_e4m3_b128")
+
+
+def weight_quant_into(w: torch.Tensor, wq: torch.Tensor, sw: torch.Tensor) -> bool:
+    """:func:`weight_quant` straight into existing storage, for instance rows of a merged layer's parameters.
+
+    ``False``, with nothing written, unless ``wq`` (e4m3, shape of ``w``) and ``sw`` (fp32, one value per 128x128 block)
+    are on ``w``'s device and can be written row by row; the caller then copies from :func:`weight_quant`'s buffers.
+    """
+    _require_cuda(w)
+    if w.dtype != torch.bfloat16 or w.dim() != 2:
+        raise TypeError("weight_quant expects a 2-D bfloat16 tensor")
+    N, K = w.shape
+    blocks = ((N + GROUP - 1) // GROUP, (K + GROUP - 1) // GROUP)
+    for t, shape, dtype in ((wq, (N, K), FP8), (sw, blocks, torch.float32)):
+        if (t.dtype != dtype or tuple(t.shape) != shape or t.device != w.device
+                or (shape[1] > 1 and t.stride(1) != 1) or (shape[0] > 1 and t.stride(0) < shape[1])):
+            return False
+    _launch_weight_quant(w, wq, sw)
+    return True
 
 
 def fp8_gemm(xq: torch.Tensor, sx: torch.Tensor, wq: torch.Tensor, sw: torch.Tensor,

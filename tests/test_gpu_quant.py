@@ -85,6 +85,55 @@ def test_weight_quant_bit_exact(ops, n, k):
     assert torch.equal(bits(wq) & 0x7F, bits(wq_ref) & 0x7F)
 
 
+@pytest.mark.parametrize("n,k,col,ldw,row,ld_wq", [
+    (256, 256, 0, 256, 128, 256),        # rows of a merged parameter, 16-byte loads
+    (130, 200, 8, 216, 0, 208),          # ragged edges, a column slice of the checkpoint tensor
+    (1, 8, 0, 8, 0, 8),                  # the smallest that 16-byte loads take
+    (129, 128, 1, 136, 128, 128),        # odd start: element by element
+    (200, 131, 0, 131, 0, 144),          # odd row length and stride
+    (128, 136, 0, 136, 0, 140),          # rows of the result not 8-byte aligned
+])
+def test_weight_quant_into_rows_bytes_equal_ieee(ops, n, k, col, ldw, row, ld_wq):
+    """Against (w / scale) in IEEE fp32, signs of zeros included, over many binades; nothing outside the rows is written."""
+    g = torch.Generator().manual_seed(n + k)
+    w = torch.randn(n, k, generator=g) * torch.exp2(torch.randint(-24, 24, (n, 1), generator=g).float())
+    w = w.masked_fill(torch.rand(n, k, generator=g) < 0.05, -0.0).to(torch.bfloat16)
+    w[:128, :128] = 0.0 if n > 200 else w[:128, :128]                       # an all-zero block
+    if n > 128:
+        w[128, 0] = float("inf")                                            # scale inf: quotients are zeros and a NaN
+    blocks = (-(-n // 128), -(-k // 128))
+    wide = torch.zeros(n, ldw, dtype=torch.bfloat16)
+    wide[:, col:col + k] = w
+    out = torch.full((row + n + 3, ld_wq), 7, dtype=torch.uint8, device="cuda")
+    scales = torch.full((row // 128 + blocks[0] + 1, blocks[1]), 7.0, device="cuda")
+    dst = out.view(torch.float8_e4m3fn)[row:row + n, :k]
+    dst_s = scales[row // 128:row // 128 + blocks[0]]
+    assert ops.weight_quant_into(wide.cuda()[:, col:col + k], dst, dst_s)
+    padded = torch.zeros(blocks[0] * 128, blocks[1] * 128)
+    padded[:n, :k] = w.float()
+    amax = padded.view(blocks[0], 128, blocks[1], 128).abs().amax(dim=(1, 3))
+    scale = amax.clamp_min(1e-10) / 448.0
+    full = scale.repeat_interleave(128, 0).repeat_interleave(128, 1)[:n, :k]
+    ref = (w.float() / full)
+    want = ref.clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8)
+    got = out.cpu()[row:row + n, :k]
+    nan = ref.isnan()
+    assert torch.equal(got[~nan], want[~nan]) and bool(((got[nan] & 0x7F) == 0x7F).all())
+    assert torch.equal(dst_s.cpu(), scale)
+    rest = out.cpu()
+    rest[row:row + n, :k] = 7
+    assert bool((rest == 7).all()) and bool((scales[row // 128 + blocks[0]:] == 7).all()) and bool((scales[:row // 128] == 7).all())
+
+
+def test_weight_quant_into_declines_what_it_cannot_write(ops):
+    w = torch.randn(128, 256, device="cuda").to(torch.bfloat16)
+    q = torch.zeros(128, 256, dtype=torch.uint8, device="cuda").view(torch.float8_e4m3fn)
+    s = torch.zeros(1, 2, device="cuda")
+    for wq, sw in ((q[:64], s), (q, s[:, :1]), (q.view(256, 128).t(), s), (q.cpu(), s), (q, s.double())):
+        assert not ops.weight_quant_into(w, wq, sw)
+    assert not q.view(torch.uint8).any() and not s.any()
+
+
 def test_quantisers_leave_status_clean(ops):
     from nano_qwen_b200 import _cabi
     torch.cuda.synchronize()
