@@ -10,7 +10,6 @@
 // Both round to bf16 exactly where the reference's eager code produces a bf16 tensor, and then apply the
 // rule of act_quant_kernel (scale = max(amax, 1e-10) / 448, q = RNE_e4m3(h / scale), IEEE divides), so that the
 // bytes equal "reference op, then activation quantiser" whenever the fp32 intermediates agree.
-// Layout: 8 lanes per 128-wide group, 16 consecutive elements per lane, like act_quant_kernel.
 #include "nq_internal.cuh"
 
 namespace nq {
@@ -64,45 +63,143 @@ __device__ __forceinline__ uint4 pack8_bf16(const float* v) {
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+__device__ __forceinline__ uint32_t bf16x2_mul(uint32_t a, uint32_t b) {
+  const __nv_bfloat162 r = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+__device__ __forceinline__ uint32_t bf16x2_one_plus(uint32_t a) {
+  const __nv_bfloat162 r = __hadd2(__float2bfloat162_rn(1.0f), *reinterpret_cast<const __nv_bfloat162*>(&a));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+__device__ __forceinline__ uint32_t bf16x2_pack(float lo, float hi) {
+  const __nv_bfloat162 r = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+// Bound by HBM for large batches (4 bytes in, 1 out per element; 12288 wide, 8192 rows: 93 us = 5.4 TB/s; products,
+// roundings and amax one value at a time took 119 us), by one lane's chain of loads, exponentials, shuffles and
+// divisions for small ones.  That is why E, the elements per lane, is 8 as long as all lanes are resident at once
+// (1 row: 1.7 us against 2.0, 256 rows of 6400: 3.8 against 4.5) and 16 beyond (512 rows of 6400: 5.4 against 6.1).
+// 40 registers (6 CTAs per SM): with 48 a batch of 256 rows of 12288 needed a second, nearly empty wave (6.5 us, now 5.2).
 // gate_up [M, 2*I] bf16 (gate = columns [0, I), up = columns [I, 2I)), row stride ld elements.
-__global__ void __launch_bounds__(256) silu_mul_quant_kernel(const __nv_bfloat16* __restrict__ gu, int64_t M, int64_t I,
-                                                             int64_t ld, uint8_t* __restrict__ xq, int64_t ld_xq,
-                                                             float* __restrict__ sx, int64_t ld_sx) {
+template <int E>
+__global__ void __launch_bounds__(256, 6) silu_mul_quant_kernel(const __nv_bfloat16* __restrict__ gu, int64_t M, int64_t I,
+                                                                int64_t ld, uint8_t* __restrict__ xq, int64_t ld_xq,
+                                                                float* __restrict__ sx, int64_t ld_sx) {
+  constexpr int L = 128 / E;                                 // lanes per group
   pdl_launch_next();   // the consumer GEMM sets up and prefetches weights meanwhile; it waits for this grid itself
   pdl_wait_prior();
   const int64_t G = (I + 127) >> 7;
   const int64_t items = M * G;
-  const int sub = threadIdx.x >> 3, l8 = threadIdx.x & 7;
-  const uint32_t mask8 = 0xFFu << (threadIdx.x & 24);
-  for (int64_t item = static_cast<int64_t>(blockIdx.x) * 32 + sub; item < items;
-       item += static_cast<int64_t>(gridDim.x) * 32) {
+  const int sub = threadIdx.x / L, l = threadIdx.x % L;
+  const uint32_t lanes = ((1u << L) - 1u) << (threadIdx.x & 31 & ~(L - 1));
+  for (int64_t item = static_cast<int64_t>(blockIdx.x) * (256 / L) + sub; item < items;
+       item += static_cast<int64_t>(gridDim.x) * (256 / L)) {
     const int64_t m = item / G, g = item - m * G;
-    const int64_t k0 = (g << 7) + (l8 << 4);
-    float a[16], b[16], h[16];
-    if (k0 < I) {                                            // I is a multiple of 16: a lane is all in or all out
+    const int64_t k0 = (g << 7) + l * E;
+    const bool in = k0 < I;                                  // I is a multiple of 16: a lane is all in or all out
+    uint32_t a[E / 2], h[E / 2], q[E / 4];
+#pragma unroll
+    for (int i = 0; i < E / 2; ++i) h[i] = 0u;
+    if (in) {
       const uint4* pg = reinterpret_cast<const uint4*>(gu + m * ld + k0);
       const uint4* pu = reinterpret_cast<const uint4*>(gu + m * ld + I + k0);
-      unpack16(__ldg(pg), __ldg(pg + 1), a);
-      unpack16(__ldg(pu), __ldg(pu + 1), b);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        // silu in fp32 with the hardware exponential and reciprocal: a few fp32 ulp, far below the bf16 rounding
-        // that follows (F.silu returns bf16; bf16 * bf16 rounds once more)
-        const float s = __fdividef(a[i], 1.0f + __expf(-a[i]));
-        h[i] = bf16_round(bf16_round(s) * b[i]);
+      for (int i = 0; i < E / 8; ++i) {
+        const uint4 g4 = __ldg(pg + i), u4 = __ldg(pu + i);
+        a[4 * i] = g4.x; a[4 * i + 1] = g4.y; a[4 * i + 2] = g4.z; a[4 * i + 3] = g4.w;
+        h[4 * i] = u4.x; h[4 * i + 1] = u4.y; h[4 * i + 2] = u4.z; h[4 * i + 3] = u4.w;
       }
-    } else {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) h[i] = 0.0f;
+      for (int i = 0; i < E / 2; ++i) {
+        // silu in fp32 with the hardware exponential and reciprocal: a few fp32 ulp, far below the bf16 rounding
+        // that follows (F.silu returns bf16; bf16 * bf16 rounds once more: the packed product is that rounding)
+        const float2 v = bf16x2_unpack(a[i]);
+        h[i] = bf16x2_mul(bf16x2_pack(__fdividef(v.x, 1.0f + __expf(-v.x)), __fdividef(v.y, 1.0f + __expf(-v.y))), h[i]);
+      }
     }
     float scale;
-    const uint4 q = quantise16(h, mask8, scale);
-    if (l8 == 0) sx[g * ld_sx + m] = scale;
-    if (k0 < I) *reinterpret_cast<uint4*>(xq + m * ld_xq + k0) = q;
+    quantise_packed<E>(h, lanes, scale, q);
+    if (l == 0) sx[g * ld_sx + m] = scale;
+    if (in) {
+      uint8_t* dst = xq + m * ld_xq + k0;
+      if constexpr (E == 16) *reinterpret_cast<uint4*>(dst) = make_uint4(q[0], q[1], q[2], q[3]);
+      else *reinterpret_cast<uint2*>(dst) = make_uint2(q[0], q[1]);
+    }
   }
 }
 
-// One CTA of 256 threads per token row.  Pass 1: x (+ residual) in fp32, sum of squares.  Pass 2 reads the row again
+// Rows of up to 8192 elements: one CTA per row at a time, 8 elements per thread.
+// Small batches are a chain of latencies between two GEMMs: all loads of a row are in flight at once, the row stays in
+// registers between the sum of squares and the quantiser, every thread forms the row's factor itself (one barrier).
+// Two passes over the row by 256 threads took 2.8 us at 4096 columns and 4.1 us at 5120 (whose last 1024 columns were a
+// second trip of a quarter of the threads); now 2.1 and 2.2 us.  Large batches are bound by HBM (7 bytes per element):
+// a CTA requests its next row before it reduces the present one; 8192 rows of 4096: 54 -> 47 us (36 us at copy rate).
+__global__ void __launch_bounds__(1024, 1) rmsnorm_row_quant_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* res_in,
+                                                                    const __nv_bfloat16* __restrict__ weight, float eps, int gemma,
+                                                                    int64_t M, int64_t H, int64_t ldx, int64_t ld_res,
+                                                                    __nv_bfloat16* res_out, __nv_bfloat16* y_out, int64_t ldy,
+                                                                    uint8_t* __restrict__ xq, int64_t ld_xq, float* __restrict__ sx,
+                                                                    int64_t ld_sx) {
+  __shared__ float warp_sum[2][32];
+  pdl_launch_next();   // the consumer GEMM sets up and prefetches weights meanwhile; it waits for this grid itself
+  const int k0 = threadIdx.x * 8, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int warps = blockDim.x >> 5;
+  const bool in = k0 < H;                                    // H is a multiple of 16
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  pdl_wait_prior();
+  int64_t m = blockIdx.x;
+  uint4 xp = zero, rp = zero;
+  // the residual may be updated in place (res_out == res_in): plain loads, before this thread's own store to the row
+  auto fetch = [&](int64_t row) {
+    if (!in) return;
+    xp = __ldg(reinterpret_cast<const uint4*>(x + row * ldx + k0));
+    if (res_in != nullptr) rp = *reinterpret_cast<const uint4*>(res_in + row * ld_res + k0);
+  };
+  fetch(m);
+  uint4 w = in ? __ldg(reinterpret_cast<const uint4*>(weight + k0)) : zero;
+  if (gemma) w = make_uint4(bf16x2_one_plus(w.x), bf16x2_one_plus(w.y), bf16x2_one_plus(w.z), bf16x2_one_plus(w.w));
+  for (int parity = 0; m < M; parity ^= 1) {
+    const uint32_t xw[4] = {xp.x, xp.y, xp.z, xp.w}, rw[4] = {rp.x, rp.y, rp.z, rp.w};
+    float2 v[4];
+    float ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[i] = bf16x2_unpack(xw[i]);
+      if (res_in != nullptr) {
+        const float2 r = bf16x2_unpack(rw[i]);
+        v[i] = make_float2(v[i].x + r.x, v[i].y + r.y);
+      }
+      ss = fmaf(v[i].x, v[i].x, ss);
+      ss = fmaf(v[i].y, v[i].y, ss);
+    }
+    const int64_t next = m + gridDim.x;
+    if (next < M) fetch(next);
+    if (res_out != nullptr && in)
+      *reinterpret_cast<uint4*>(res_out + m * ld_res + k0) = make_uint4(bf16x2_pack(v[0].x, v[0].y), bf16x2_pack(v[1].x, v[1].y),
+                                                                        bf16x2_pack(v[2].x, v[2].y), bf16x2_pack(v[3].x, v[3].y));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
+    if (lane == 0) warp_sum[parity][warp] = ss;
+    __syncthreads();                                         // two sets of sums: the next row's cannot overtake a reader
+    float t = lane < warps ? warp_sum[parity][lane] : 0.0f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
+    const float rstd = __fdiv_rn(1.0f, __fsqrt_rn(__fdiv_rn(t, static_cast<float>(H)) + eps));
+    const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+    uint32_t h[4], q[2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)                              // x.to(orig_dtype), then bf16 tensor * bf16 tensor
+      h[i] = in ? bf16x2_mul(bf16x2_pack(v[i].x * rstd, v[i].y * rstd), ww[i]) : 0u;
+    if (y_out != nullptr && in) *reinterpret_cast<uint4*>(y_out + m * ldy + k0) = make_uint4(h[0], h[1], h[2], h[3]);
+    float scale;
+    quantise_packed<8>(h, 0xFFFFu << (lane & 16), scale, q);
+    if ((lane & 15) == 0 && in) sx[static_cast<int64_t>(threadIdx.x >> 4) * ld_sx + m] = scale;
+    if (in) *reinterpret_cast<uint2*>(xq + m * ld_xq + k0) = make_uint2(q[0], q[1]);
+    m = next;
+  }
+}
+
+// Rows of more than 8192 elements.  One CTA of 256 threads per token row.  Pass 1: x (+ residual) in fp32, sum of squares.  Pass 2 reads the row again
 // (from L1/L2), writes the new residual, normalises, rounds to bf16, multiplies by the weight in bf16 and quantises.
 // (Keeping the row in registers between the passes was measured slower: 80 registers halve the CTAs per SM.)
 __global__ void __launch_bounds__(256) rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* res_in,
@@ -214,8 +311,11 @@ int nq_silu_mul_quant_e4m3_g128(const void* gate_up, int64_t M, int64_t I, int64
   const int st = ensure_init(&ctx);
   if (st != NQ_OK) return st;
   const int64_t items = M * ((I + 127) / 128);
-  int64_t blocks = (items + 31) / 32;
-  const int64_t cap = static_cast<int64_t>(ctx->sm_count) * 16;
+  // 8 elements per lane while the CTAs of 16 groups fit the GPU at once (6 per SM), else 16 (see the kernel)
+  const bool narrow = items <= static_cast<int64_t>(ctx->sm_count) * 96;
+  const int64_t per_block = narrow ? 16 : 32;
+  int64_t blocks = (items + per_block - 1) / per_block;
+  const int64_t cap = static_cast<int64_t>(ctx->sm_count) * 24;
   if (blocks > cap) blocks = cap;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(blocks));
@@ -226,7 +326,7 @@ int nq_silu_mul_quant_e4m3_g128(const void* gate_up, int64_t M, int64_t I, int64
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, silu_mul_quant_kernel, static_cast<const __nv_bfloat16*>(gate_up), M, I,
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, narrow ? silu_mul_quant_kernel<8> : silu_mul_quant_kernel<16>, static_cast<const __nv_bfloat16*>(gate_up), M, I,
                                            ld, static_cast<uint8_t*>(xq), ld_xq, sx, ld_sx);
   count_launch();
   return check_cuda(e);
@@ -259,6 +359,19 @@ int nq_rmsnorm_quant_e4m3_g128(const void* x, const void* residual_in, const voi
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  if (H <= 8192) {
+    const int64_t threads = (H + 255) / 256 * 32;
+    // as many CTAs as are resident at once (63 registers: 1024 threads per SM); asking for 1536 threads per SM cost 5-10 %
+    const int64_t slots = ctx->sm_count * (1024 / threads);
+    cfg.gridDim = dim3(static_cast<unsigned>(M < slots ? M : slots));
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    const cudaError_t e = cudaLaunchKernelEx(
+        &cfg, rmsnorm_row_quant_kernel, static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(residual_in),
+        static_cast<const __nv_bfloat16*>(weight), eps, gemma, M, H, ldx, ld_res, static_cast<__nv_bfloat16*>(residual_out),
+        static_cast<__nv_bfloat16*>(y_out), ldy, static_cast<uint8_t*>(xq), ld_xq, sx, ld_sx);
+    count_launch();
+    return check_cuda(e);
+  }
   const cudaError_t e = cudaLaunchKernelEx(
       &cfg, rmsnorm_quant_kernel, static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(residual_in),
       static_cast<const __nv_bfloat16*>(weight), eps, gemma, H, ldx, ld_res, static_cast<__nv_bfloat16*>(residual_out),

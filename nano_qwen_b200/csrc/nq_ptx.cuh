@@ -445,4 +445,34 @@ __device__ __forceinline__ uint32_t pack4_e4m3(float a, float b, float c, float 
 }
 
 
+__device__ __forceinline__ float2 bf16x2_unpack(uint32_t w) {
+  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+}
+
+// E bf16 values of one lane, as E / 2 packed pairs -> amax over the 128 / E lanes of the group -> scale -> E e4m3 bytes.
+template <int E>
+__device__ __forceinline__ void quantise_packed(const uint32_t (&h)[E / 2], uint32_t lanes, float& scale, uint32_t (&q)[E / 4]) {
+  uint32_t m2 = 0u;                                          // a maximum of bf16 values is exact
+#pragma unroll
+  for (int i = 0; i < E / 2; ++i) m2 = bf16x2_absmax(m2, h[i]);
+  float amax = fmaxf(bf16_bits_to_float(m2 & 0xFFFFu), bf16_bits_to_float(m2 >> 16));
+#pragma unroll
+  for (int o = 1; o < 128 / E; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(lanes, amax, o));
+  scale = __fdiv_rn(fmaxf(amax, 1e-10f), 448.0f);
+  const ExactDivider div(scale);
+  if (!div.slow) {
+#pragma unroll
+    for (int i = 0; i < E / 4; ++i) {
+      const float2 a = div.fast2(bf16x2_unpack(h[2 * i])), b = div.fast2(bf16x2_unpack(h[2 * i + 1]));
+      q[i] = pack4_e4m3(a.x, a.y, b.x, b.y);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < E / 4; ++i) {
+      const float2 a = bf16x2_unpack(h[2 * i]), b = bf16x2_unpack(h[2 * i + 1]);
+      q[i] = pack4_e4m3(__fdiv_rn(a.x, scale), __fdiv_rn(a.y, scale), __fdiv_rn(b.x, scale), __fdiv_rn(b.y, scale));
+    }
+  }
+}
+
 }  // namespace nq

@@ -112,6 +112,50 @@ def test_rmsnorm_quant_matches_oracle(ops, m, h, gemma):
     check_quantised(xq, sx, ref)
 
 
+@pytest.mark.parametrize("h", [16, 272, 5120, 8176, 8192, 8208])
+def test_rmsnorm_quant_many_rows_in_place(ops, h):
+    """More rows than CTAs (each takes several, the next one requested early), the residual updated in place, strided
+    rows; 8192 columns fill a CTA, 8208 take the two-pass kernel.  Row by row equal to calls with one row each."""
+    from nano_qwen_b200 import _cabi
+    m, pad = 148 * max(1, 1024 // (-(-h // 256) * 32)) + 151, 16
+    gen = torch.Generator(device="cuda").manual_seed(h)
+    x = torch.randn(m, h + pad, generator=gen, device="cuda").to(torch.bfloat16)
+    res = torch.randn(m, h + pad, generator=gen, device="cuda").to(torch.bfloat16)
+    w = torch.randn(h, generator=gen, device="cuda").to(torch.bfloat16)
+    groups = -(-h // 128)
+    xq = torch.empty(m, h, dtype=torch.uint8, device="cuda")
+    sx = torch.empty(groups, m, dtype=torch.float32, device="cuda")
+    new = res.clone()
+    st = _cabi.lib().nq_rmsnorm_quant_e4m3_g128(x.data_ptr(), new.data_ptr(), w.data_ptr(), 1e-6, 1, m, h, h + pad, h + pad,
+                                                new.data_ptr(), None, 0, xq.data_ptr(), h, sx.data_ptr(), m,
+                                                torch.cuda.current_stream().cuda_stream)
+    assert st == 0
+    want = torch.cat([res[:, :h].float().add(x[:, :h].float()).to(torch.bfloat16), res[:, h:]], 1)
+    assert torch.equal(new.view(torch.int16), want.view(torch.int16))
+    for r in (0, 1, 147, 148, m // 2, m - 2, m - 1):
+        q1, s1, _, _ = ops.rmsnorm_quant(x[r:r + 1, :h], w, 1e-6, res[r:r + 1, :h], gemma=True)
+        assert torch.equal(q1.view(torch.uint8)[0], xq[r]) and torch.equal(s1[0], sx[:, r])
+    rows = torch.tensor([0, 149, m - 1])
+    ref, _ = R.rms_norm(x[rows.cuda(), :h].cpu(), w.cpu(), 1e-6, res[rows.cuda(), :h].cpu(), gemma=True)
+    if h > 16:                                              # 48 bytes are too few for a share of equal ones
+        check_quantised(xq[rows.cuda()].view(torch.float8_e4m3fn), sx[:, rows.cuda()].t(), ref)
+
+
+@pytest.mark.parametrize("m", [1, 888, 889])
+def test_silu_mul_quant_narrow_and_wide_lanes(ops, m):
+    """Groups of 8 elements per lane up to one wave of CTAs (148 SMs: 14208 groups = 888 rows of 16), of 16 beyond: the same
+    bytes either side, rows that end inside a group, and the values the arithmetic has to carry through."""
+    inter = 16 * 128 - 112
+    gen = torch.Generator().manual_seed(5)
+    gu = (torch.randn(889, 2 * inter, generator=gen) * 4.0).to(torch.bfloat16)
+    gu[0, :4] = torch.tensor([-0.0, 90.0, -90.0, 1e-30])
+    gu[0, inter:inter + 4] = torch.tensor([1.0, -0.0, 3.0, 2.0])
+    xq, sx = ops.silu_mul_quant(gu[:m].cuda())
+    check_quantised(xq, sx, R.silu_and_mul(gu[:m]))
+    wide_q, wide_s = ops.silu_mul_quant(gu.cuda())
+    assert torch.equal(xq.view(torch.uint8), wide_q.view(torch.uint8)[:m]) and torch.equal(sx, wide_s[:m])
+
+
 def test_full_size_producers_sampled_rows(ops):
     """Prefill-sized inputs (larger than L2): 48 sampled token rows against the oracle."""
     gen = torch.Generator(device="cuda").manual_seed(31)
