@@ -11,93 +11,71 @@
 namespace nq {
 
 // ------------------------------------------------------------------------- //
-// Activation quantiser.  One 8-lane sub-warp per (token, group); each lane owns
-// 16 consecutive elements: two 128-bit loads, one 128-bit store.  A warp covers
-// four consecutive groups = 1 KiB of contiguous input when the groups share a row.
-// amax over the sub-warp by three xor-shuffles.
-// VEC=false is the ragged/unaligned variant (element-wise guarded accesses).
+// Activation quantiser.  128 / E lanes per (token, group), E consecutive elements per lane; a warp covers 1 KiB (E = 16) or
+// 512 B (E = 8) of contiguous input when the groups share a row.
+// VEC: 16-byte loads.  E = 16 for whole groups (K a multiple of 128), E = 8 for rows that end inside a group but on a
+// multiple of 8, where a lane is inside the row or outside it as a whole (8192 rows of 1096: 36 us element by element,
+// 13 us so; 8 rows: 3.1 -> 1.5 us).
+// VEC = false is the variant for odd sizes and unaligned rows (element-wise guarded accesses).
 // ------------------------------------------------------------------------- //
-template <bool VEC>
-__global__ void __launch_bounds__(256) act_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t M, int64_t K,
+template <int E, bool VEC>
+__global__ void __launch_bounds__(256, E == 8 ? 6 : 1) act_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t M, int64_t K,
                                                         int64_t ldx, uint8_t* __restrict__ xq, int64_t ld_xq,
                                                         float* __restrict__ sx, int64_t ld_sx) {
+  constexpr int L = 128 / E, kGroups = 256 / L;
   // Let the GEMM that follows start at once: its set-up and its first weight tiles do not depend on this kernel (it
   // waits for this grid's completion itself, with griddepcontrol.wait, before it touches xq / sx).
   pdl_launch_next();
   pdl_wait_prior();
   const int64_t G = (K + 127) >> 7;
   const int64_t items = M * G;
-  const int sub = threadIdx.x >> 3;   // 0..31 sub-warp within the block
-  const int l8 = threadIdx.x & 7;     // lane within the sub-warp
-  // Grid-stride loop; the aligned variant requests the next item's 32 bytes before it converts the current one.
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * 32;
-  int64_t item = static_cast<int64_t>(blockIdx.x) * 32 + sub;
-  uint4 na = make_uint4(0u, 0u, 0u, 0u), nb = na;
-  if (VEC && item < items) {
-    const int64_t m = item / G, g = item - m * G;
-    const uint4* src = reinterpret_cast<const uint4*>(x + m * ldx + (g << 7) + (l8 << 4));
-    na = __ldg(src);
-    nb = __ldg(src + 1);
-  }
+  const int sub = threadIdx.x / L, l = threadIdx.x % L;
+  // sub-warps of one warp may leave the loop at different items: mask = own lanes
+  const uint32_t lanes = ((1u << L) - 1u) << (threadIdx.x & 31 & ~(L - 1));
+  // Grid-stride loop; the aligned variant requests the next item's elements before it converts the current ones.
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * kGroups;
+  int64_t item = static_cast<int64_t>(blockIdx.x) * kGroups + sub;
+  uint4 ahead[E / 8];
+  auto fetch = [&](int64_t it) {
+    const int64_t m = it / G, k = ((it - m * G) << 7) + l * E;
+#pragma unroll
+    for (int i = 0; i < E / 8; ++i)
+      ahead[i] = (E == 16 || k < K) ? __ldg(reinterpret_cast<const uint4*>(x + m * ldx + k) + i) : make_uint4(0u, 0u, 0u, 0u);
+  };
+  if (VEC && item < items) fetch(item);
   for (; item < items; item += stride) {
     const int64_t m = item / G;
     const int64_t g = item - m * G;
-    const int64_t k0 = (g << 7) + (l8 << 4);
-    // the 16 elements as 8 words of two bf16 each (element 2i in the low half of word i)
-    uint32_t w[8];
+    const int64_t k0 = (g << 7) + l * E;
+    uint32_t w[E / 2], q[E / 4];                             // word i: elements 2i (low half) and 2i + 1
     if (VEC) {
-      w[0] = na.x; w[1] = na.y; w[2] = na.z; w[3] = na.w; w[4] = nb.x; w[5] = nb.y; w[6] = nb.z; w[7] = nb.w;
-      const int64_t nxt = item + stride;
-      if (nxt < items) {
-        const int64_t m1 = nxt / G, g1 = nxt - m1 * G;
-        const uint4* src = reinterpret_cast<const uint4*>(x + m1 * ldx + (g1 << 7) + (l8 << 4));
-        na = __ldg(src);
-        nb = __ldg(src + 1);
+#pragma unroll
+      for (int i = 0; i < E / 8; ++i) {
+        w[4 * i] = ahead[i].x; w[4 * i + 1] = ahead[i].y; w[4 * i + 2] = ahead[i].z; w[4 * i + 3] = ahead[i].w;
       }
+      if (item + stride < items) fetch(item + stride);
     } else {
       const unsigned short* src = reinterpret_cast<const unsigned short*>(x + m * ldx);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
+      for (int i = 0; i < E / 2; ++i) {
         const uint32_t lo = (k0 + 2 * i < K) ? src[k0 + 2 * i] : 0u;
         const uint32_t hi = (k0 + 2 * i + 1 < K) ? src[k0 + 2 * i + 1] : 0u;
         w[i] = lo | (hi << 16);
       }
     }
-    // amax on the packed pairs (a maximum of bf16 values is exact), then across the pair and the sub-warp
-    uint32_t m2 = bf16x2_absmax(w[0], w[1]);
-#pragma unroll
-    for (int i = 2; i < 8; i += 2) m2 = bf16x2_absmax(m2, bf16x2_absmax(w[i], w[i + 1]));
-    float amax = fmaxf(bf16_bits_to_float(m2 & 0xFFFFu), bf16_bits_to_float(m2 >> 16));
-    // sub-warps of one warp may leave the loop at different items: mask = own 8 lanes
-    const uint32_t mask8 = 0xFFu << (threadIdx.x & 24);
-    amax = fmaxf(amax, __shfl_xor_sync(mask8, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(mask8, amax, 2));
-    amax = fmaxf(amax, __shfl_xor_sync(mask8, amax, 4));
-    const float scale = __fdiv_rn(fmaxf(amax, 1e-10f), 448.0f);
-    if (l8 == 0) sx[g * ld_sx + m] = scale;
-    const ExactDivider div(scale);
-    uint32_t qw[4];
-    if (!div.slow) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 a = div.fast2(make_float2(__uint_as_float(w[2 * i] << 16), __uint_as_float(w[2 * i] & 0xFFFF0000u)));
-        const float2 b = div.fast2(make_float2(__uint_as_float(w[2 * i + 1] << 16), __uint_as_float(w[2 * i + 1] & 0xFFFF0000u)));
-        qw[i] = pack4_e4m3(a.x, a.y, b.x, b.y);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        qw[i] = pack4_e4m3(__fdiv_rn(__uint_as_float(w[2 * i] << 16), scale), __fdiv_rn(__uint_as_float(w[2 * i] & 0xFFFF0000u), scale),
-                           __fdiv_rn(__uint_as_float(w[2 * i + 1] << 16), scale), __fdiv_rn(__uint_as_float(w[2 * i + 1] & 0xFFFF0000u), scale));
-      }
-    }
-    const uint4 q = make_uint4(qw[0], qw[1], qw[2], qw[3]);
+    float scale;
+    quantise_packed<E>(w, lanes, scale, q);
+    if (l == 0) sx[g * ld_sx + m] = scale;
+    uint8_t* dst = xq + m * ld_xq + k0;
     if (VEC) {
-      *reinterpret_cast<uint4*>(xq + m * ld_xq + k0) = q;
+      if (E == 16 || k0 < K) {
+        if constexpr (E == 16) *reinterpret_cast<uint4*>(dst) = make_uint4(q[0], q[1], q[2], q[3]);
+        else *reinterpret_cast<uint2*>(dst) = make_uint2(q[0], q[1]);
+      }
     } else {
 #pragma unroll
-      for (int i = 0; i < 16; ++i)
-        if (k0 + i < K) xq[m * ld_xq + k0 + i] = static_cast<uint8_t>(qw[i >> 2] >> ((i & 3) * 8));
+      for (int i = 0; i < E; ++i)
+        if (k0 + i < K) dst[i] = static_cast<uint8_t>(q[i >> 2] >> ((i & 3) * 8));
     }
   }
 }
@@ -192,12 +170,15 @@ int launch_act_quant(const void* x, int64_t M, int64_t K, int64_t ldx, void* xq,
   const int64_t G = (K + 127) / 128;
   const int64_t items = M * G;
   if (items == 0) return NQ_OK;
-  const bool vec = (K % 128 == 0) && (ldx % 8 == 0) && (ld_xq % 16 == 0) &&
-                   (reinterpret_cast<uintptr_t>(x) % 16 == 0) && (reinterpret_cast<uintptr_t>(xq) % 16 == 0);
-  int64_t blocks = (items + 31) / 32;
   DeviceCtx* ctx = nullptr;
   const int st = ensure_init(&ctx);
   if (st != NQ_OK) return st;
+  const bool vec8 = (K % 8 == 0) && (ldx % 8 == 0) && (ld_xq % 8 == 0) &&
+                    (reinterpret_cast<uintptr_t>(x) % 16 == 0) && (reinterpret_cast<uintptr_t>(xq) % 8 == 0);
+  // whole groups: 16 elements per lane at every size (with 8, 144 rows of 4096 took 2.3 us against 1.7)
+  const bool vec16 = vec8 && (K % 128 == 0) && (ld_xq % 16 == 0) && (reinterpret_cast<uintptr_t>(xq) % 16 == 0);
+  const int64_t per_block = vec8 && !vec16 ? 16 : 32;
+  int64_t blocks = (items + per_block - 1) / per_block;
   // grid-stride loop over at most 32 CTAs per SM (several waves smooth the tail; measured equal from 10 to 64)
   const int64_t cap = static_cast<int64_t>(ctx->sm_count) * 32;
   if (blocks > cap) blocks = cap;
@@ -212,8 +193,8 @@ int launch_act_quant(const void* x, int64_t M, int64_t K, int64_t ldx, void* xq,
   cfg.numAttrs = pdl ? 1 : 0;
   auto* xp = static_cast<const __nv_bfloat16*>(x);
   auto* qp = static_cast<uint8_t*>(xq);
-  cudaError_t e = vec ? cudaLaunchKernelEx(&cfg, act_quant_kernel<true>, xp, M, K, ldx, qp, ld_xq, sx, ld_sx)
-                      : cudaLaunchKernelEx(&cfg, act_quant_kernel<false>, xp, M, K, ldx, qp, ld_xq, sx, ld_sx);
+  const auto kernel = vec16 ? act_quant_kernel<16, true> : vec8 ? act_quant_kernel<8, true> : act_quant_kernel<16, false>;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, xp, M, K, ldx, qp, ld_xq, sx, ld_sx);
   count_launch();
   return check_cuda(e);
 }

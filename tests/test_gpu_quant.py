@@ -34,6 +34,27 @@ def test_act_quant_bit_exact(ops, m, k):
     assert torch.equal(bits(xq)[nz], bits(xq_ref)[nz])
 
 
+@pytest.mark.parametrize("m,k,col", [(1, 8, 0), (301, 1096, 0), (3000, 136, 0), (17, 1096, 8), (17, 1096, 4), (9, 1100, 0)])
+def test_act_quant_rows_that_end_inside_a_group(ops, m, k, col):
+    """Multiples of 8 with 16-byte loads; a start that is not 16-byte aligned and other lengths element by element.
+    The bytes between a row's end and the next row are left alone."""
+    from nano_qwen_b200 import _cabi
+    g = torch.Generator().manual_seed(k + col)
+    wide = (torch.randn(m, k + 16, generator=g) * 8.0).to(torch.bfloat16)
+    x = wide[:, col:col + k]
+    xq_ref, sx_ref = S.quantize_act_group128(x)
+    ld = (k + 15) // 16 * 16 + 16
+    xq = torch.full((m, ld), 7, dtype=torch.uint8, device="cuda")
+    sx = torch.empty(sx_ref.shape[1], m, device="cuda")
+    xd = wide.cuda()[:, col:col + k]
+    st = _cabi.lib().nq_act_quant_e4m3_g128(xd.data_ptr(), m, k, xd.stride(0), xq.data_ptr(), ld, sx.data_ptr(), m,
+                                            torch.cuda.current_stream().cuda_stream)
+    assert st == 0
+    assert torch.equal(bits(sx.t().contiguous()), bits(sx_ref))
+    assert torch.equal(xq[:, :k].cpu() & 0x7F, bits(xq_ref) & 0x7F)
+    assert bool((xq[:, k:] == 7).all())
+
+
 def test_act_quant_bit_exact_over_many_scales(ops):
     """16 M elements, per-row magnitudes from 2^-60 to 2^60: the reciprocal-based exact division agrees
     with the IEEE divide of the oracle on every byte."""
