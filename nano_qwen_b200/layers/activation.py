@@ -30,5 +30,5 @@ class SiluAndMul(nn.Module):
             raise RuntimeError(f"SiluAndMul(emit_fp8=True) needs a CUDA bfloat16 tensor, got {x.device.type} {x.dtype}: "
                                "there is no CPU fallback (construct it with emit_fp8=False for the eager op)")
         inter = x.shape[-1] // 2
-        xq, sx = ops.silu_mul_quant(x.reshape(-1, x.shape[-1]))
+        xq, sx = ops.silu_mul_quant(x if x.dim() == 2 and inter > 0 else x.reshape(-1, x.shape[-1]))
         return QuantizedActivation(xq, sx, (*x.shape[:-1], inter))

@@ -45,10 +45,11 @@ class _NormBase(nn.Module):
             raise RuntimeError(f"{type(self).__name__}(emit_fp8=True) needs a CUDA bfloat16 tensor, got {x.device.type} "
                                f"{x.dtype}: there is no CPU fallback (construct it with emit_fp8=False for the eager op)")
         H = x.shape[-1]
-        res2 = residual.reshape(-1, H) if residual is not None else None
-        xq, sx, new_res, _ = ops.rmsnorm_quant(x.reshape(-1, H), self.weight, self.eps, res2, gemma=self.gemma)
+        flat = x.dim() == 2 and H > 0
+        res2 = residual if residual is None or (flat and residual.shape == x.shape) else residual.reshape(-1, H)
+        xq, sx, new_res, _ = ops.rmsnorm_quant(x if flat else x.reshape(-1, H), self.weight, self.eps, res2, gemma=self.gemma)
         out = QuantizedActivation(xq, sx, x.shape)
-        return out if residual is None else (out, new_res.view(x.shape))
+        return out if residual is None else (out, new_res if flat else new_res.view(x.shape))
 
 
 class RMSNorm(_NormBase):

@@ -124,7 +124,7 @@ class LinearBase(nn.Module):
     def _linear(self, x, bias: torch.Tensor | None) -> torch.Tensor:
         if isinstance(x, QuantizedActivation):       # a fused producer already quantised it: GEMM only
             y = ops.fp8_gemm(x.xq, x.sx, self.weight, self.weight_scale_inv, bias)
-            return y.view(*x.shape[:-1], y.shape[-1])
+            return y if len(x.shape) == 2 else y.view(*x.shape[:-1], y.shape[-1])
         return ops.fp8_linear(x, self.weight, self.weight_scale_inv, bias)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:

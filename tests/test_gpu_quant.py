@@ -55,6 +55,26 @@ def test_act_quant_rows_that_end_inside_a_group(ops, m, k, col):
     assert bool((xq[:, k:] == 7).all())
 
 
+@pytest.mark.parametrize("m,k", [(1, 8), (7, 200), (8, 256)])
+def test_quantised_layout_and_leading_dimensions(ops, m, k):
+    """Row strides are multiples of 16 bytes, scales are K-group major; a 3-D input gives what its 2-D view gives, on a
+    stream of its own too."""
+    x = torch.randn(2, m, k, device="cuda").to(torch.bfloat16)
+    w = torch.randn(24, k, device="cuda").to(torch.bfloat16)
+    xq, sx = ops.act_quant(x[0])
+    assert xq.stride() == ((k + 15) // 16 * 16, 1) and sx.stride() == (1, (m + 3) // 4 * 4)
+    wq, sw = ops.weight_quant(w)
+    flat = ops.fp8_linear(x.view(2 * m, k), wq, sw)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        lead = ops.fp8_linear(x, wq, sw)
+        assert ops._stream() == stream.cuda_stream
+    stream.synchronize()
+    assert lead.shape == (2, m, 24) and torch.equal(lead.view(2 * m, 24), flat)
+    assert torch.equal(ops.fp8_gemm(xq, sx, wq, sw), flat[:m])
+
+
 def test_act_quant_bit_exact_over_many_scales(ops):
     """16 M elements, per-row magnitudes from 2^-60 to 2^60: the reciprocal-based exact division agrees
     with the IEEE divide of the oracle on every byte."""
