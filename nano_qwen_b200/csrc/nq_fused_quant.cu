@@ -130,20 +130,21 @@ __global__ void __launch_bounds__(256, 6) silu_mul_quant_kernel(const __nv_bfloa
 
 // Rows of up to 8192 elements: one CTA per row at a time, 8 elements per thread.
 // Small batches are a chain of latencies between two GEMMs: all loads of a row are in flight at once, the row stays in
-// registers between the sum of squares and the quantiser, every thread forms the row's factor itself (one barrier).
+// registers between the sum of squares and the quantiser, every thread forms the row's factor itself.
 // Two passes over the row by 256 threads took 2.8 us at 4096 columns and 4.1 us at 5120 (whose last 1024 columns were a
-// second trip of a quarter of the threads); now 2.1 and 2.2 us.  Large batches are bound by HBM (7 bytes per element):
-// a CTA requests its next row before it reduces the present one; 8192 rows of 4096: 54 -> 47 us (36 us at copy rate).
+// second trip of a quarter of the threads); now 2.2 and 2.4 us.  Large batches are bound by HBM (7 bytes per element):
+// a CTA requests its next row before it reduces the present one; 8192 rows of 4096: 54 -> 50 us (36 us at copy rate).
 __global__ void __launch_bounds__(1024, 1) rmsnorm_row_quant_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* res_in,
                                                                     const __nv_bfloat16* __restrict__ weight, float eps, int gemma,
                                                                     int64_t M, int64_t H, int64_t ldx, int64_t ld_res,
                                                                     __nv_bfloat16* res_out, __nv_bfloat16* y_out, int64_t ldy,
                                                                     uint8_t* __restrict__ xq, int64_t ld_xq, float* __restrict__ sx,
                                                                     int64_t ld_sx) {
-  __shared__ float warp_sum[2][32];
+  __shared__ float part[256];
+  __shared__ float warp_sum[8];
   pdl_launch_next();   // the consumer GEMM sets up and prefetches weights meanwhile; it waits for this grid itself
   const int k0 = threadIdx.x * 8, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int warps = blockDim.x >> 5;
+  const int strips = min(static_cast<int>(blockDim.x) >> 1, 256);
   const bool in = k0 < H;                                    // H is a multiple of 16
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   pdl_wait_prior();
@@ -158,10 +159,10 @@ __global__ void __launch_bounds__(1024, 1) rmsnorm_row_quant_kernel(const __nv_b
   fetch(m);
   uint4 w = in ? __ldg(reinterpret_cast<const uint4*>(weight + k0)) : zero;
   if (gemma) w = make_uint4(bf16x2_one_plus(w.x), bf16x2_one_plus(w.y), bf16x2_one_plus(w.z), bf16x2_one_plus(w.w));
-  for (int parity = 0; m < M; parity ^= 1) {
+  if (threadIdx.x < 8) warp_sum[threadIdx.x] = 0.0f;         // those of strips that a short row does not have stay zero
+  while (m < M) {
     const uint32_t xw[4] = {xp.x, xp.y, xp.z, xp.w}, rw[4] = {rp.x, rp.y, rp.z, rp.w};
     float2 v[4];
-    float ss = 0.0f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       v[i] = bf16x2_unpack(xw[i]);
@@ -169,21 +170,45 @@ __global__ void __launch_bounds__(1024, 1) rmsnorm_row_quant_kernel(const __nv_b
         const float2 r = bf16x2_unpack(rw[i]);
         v[i] = make_float2(v[i].x + r.x, v[i].y + r.y);
       }
-      ss = fmaf(v[i].x, v[i].x, ss);
-      ss = fmaf(v[i].y, v[i].y, ss);
     }
     const int64_t next = m + gridDim.x;
     if (next < M) fetch(next);
     if (res_out != nullptr && in)
       *reinterpret_cast<uint4*>(res_out + m * ld_res + k0) = make_uint4(bf16x2_pack(v[0].x, v[0].y), bf16x2_pack(v[1].x, v[1].y),
                                                                         bf16x2_pack(v[2].x, v[2].y), bf16x2_pack(v[3].x, v[3].y));
+    // Sum of squares in the order of the two-pass kernel below, which does not depend on how many threads share a row:
+    // 256 strips, each adding its 16 elements one by one and then those 4096 further on, a tree over 32 strips, the 8
+    // trees one after the other.  A strip is two threads; the second continues from the first one's sum.  (Another order
+    // moves the row's factor by a bit, a bf16 value with it, and two layers later most e4m3 values of the row by a step.)
+    auto add_squares = [&](float ss) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
-    if (lane == 0) warp_sum[parity][warp] = ss;
-    __syncthreads();                                         // two sets of sums: the next row's cannot overtake a reader
-    float t = lane < warps ? warp_sum[parity][lane] : 0.0f;
+      for (int i = 0; i < 4; ++i) {
+        ss = fmaf(v[i].x, v[i].x, ss);
+        ss = fmaf(v[i].y, v[i].y, ss);
+      }
+      return ss;
+    };
+    auto add_strip = [&](float from) {
+      const float first = add_squares(from);
+      const float both = add_squares(__shfl_up_sync(0xFFFFFFFFu, first, 1));
+      if (lane & 1) part[(threadIdx.x & 511) >> 1] = both;
+    };
+    if (threadIdx.x < 512) add_strip(0.0f);
+    __syncthreads();
+    if (blockDim.x > 512) {
+      if (threadIdx.x >= 512) add_strip(part[(threadIdx.x & 511) >> 1]);
+      __syncthreads();
+    }
+    if (warp * 32 < strips) {
+      float ss = threadIdx.x < strips ? part[threadIdx.x] : 0.0f;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
+      if (lane == 0) warp_sum[warp] = ss;
+    }
+    __syncthreads();
+    float t = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t += warp_sum[i];
     const float rstd = __fdiv_rn(1.0f, __fsqrt_rn(__fdiv_rn(t, static_cast<float>(H)) + eps));
     const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
     uint32_t h[4], q[2];
