@@ -161,14 +161,18 @@ int gemm_dispatch(const GemmArgs& a, int algo) {
   DeviceCtx* ctx = nullptr;
   st = ensure_init(&ctx);
   if (st != NQ_OK) return st;
-  // Measured crossover on B200 (CUDA graph, 8B layer shapes): weight rows on the lanes up to 64 tokens; at 128 tokens
-  // the token-lane kernel with 128-wide tiles is ahead (71 us against 76 us for the four linears of a layer).
+  // Measured crossover on B200 (CUDA graph, 8B layer shapes): weight rows on the lanes up to 64 tokens; at 72 tokens the
+  // token-lane kernel is ahead (65 us against 73 us for the four linears of a layer).
   // Prefill-sized launches with at least two rounds of 256 x 256 tiles go to the CTA-pair kernel: alone it runs
   // level with the single-CTA kernel (2.0-2.1 PFLOP/s), inside a long power-capped step it is 1-2 % ahead
   // (a third fewer operand bytes cross the L2 -> SM path; three interleaved runs of the 36-layer step each).
+  // In between, rounds of tiles decide (pick_token_tile): the four linears of an 8B layer take 171 us against 180 with
+  // the pair kernel left out (520 tokens), 204 / 208 (777), 217 / 228 (1024), 309 / 321 (1536).  A caller's K split goes
+  // to the kernels that can split.
   if (algo == NQ_ALGO_AUTO) {
-    algo = (a.M <= 64) ? NQ_ALGO_WEIGHT_LANE : NQ_ALGO_TOKEN_LANE;
-    if (a.M >= 2048 && ((a.M + 255) / 256) * ((a.N + 255) / 256) >= ctx->sm_count) algo = NQ_ALGO_TOKEN_PAIR;
+    if (a.M <= 64) algo = NQ_ALGO_WEIGHT_LANE;
+    else if (a.M >= 2048 && ((a.M + 255) / 256) * ((a.N + 255) / 256) >= ctx->sm_count) algo = NQ_ALGO_TOKEN_PAIR;
+    else algo = pick_token_tile(a.M, a.N, ctx->sm_count, a.split_k <= 1) == TokenTile::kPair ? NQ_ALGO_TOKEN_PAIR : NQ_ALGO_TOKEN_LANE;
   }
   if (algo == NQ_ALGO_TOKEN_LANE) return launch_gemm_token_lane(a, ctx, 0);
   if (algo == NQ_ALGO_TOKEN_LANE_128) return launch_gemm_token_lane(a, ctx, 128);

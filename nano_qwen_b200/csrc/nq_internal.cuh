@@ -47,6 +47,8 @@ struct GemmArgs {
   cudaStream_t stream;
   bool pdl;
 };
+enum class TokenTile { k128, k256, kPair };
+TokenTile pick_token_tile(int64_t M, int64_t N, int sm_count, bool pairs);   // which kernel, for more than 64 tokens
 int launch_gemm_token_lane(const GemmArgs& a, DeviceCtx* ctx, int tile_n);   // tile_n: 0 = choose, else 128/192/256
 int launch_gemm_weight_lane(const GemmArgs& a, DeviceCtx* ctx);
 int launch_gemm_token_pair(const GemmArgs& a, DeviceCtx* ctx, int tile_n);   // 256 x tile_n tiles on CTA pairs (cta_group::2)

@@ -217,3 +217,27 @@ def test_status_block_clean_after_all_gemms(ops):
     from nano_qwen_b200 import _cabi
     torch.cuda.synchronize()
     assert _cabi.device_status()["code"] == 0
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (520, 4096 + 8, 136),       # one round of 256 x 256 pair tiles, M and N ragged
+    (777, 6144, 256),           # three rounds of 128-wide tiles
+    (777, 24576, 128),          # five rounds of 256-wide tiles
+    (1281, 4096 - 8, 384),      # one row past a pair tile
+    (2047, 1000, 200),
+])
+def test_auto_between_decode_and_prefill_agrees_with_every_kernel(ops, m, n, k):
+    """The rule by rounds of tiles sends these to different kernels; unsplit, all of them add the K-tiles in one order, so
+    the bits agree, and rows whose stride allows no bulk stores take the same route."""
+    case = make_case(m, n, k, seed=m + n, bias=True)
+    y = run_gemm(ops, case, ops.ALGO_AUTO, split_k=1)
+    for algo in (ops.ALGO_TOKEN_LANE_128, ops.ALGO_TOKEN_LANE_256, ops.ALGO_TOKEN_PAIR):
+        assert torch.equal(run_gemm(ops, case, algo, split_k=1).view(torch.int16), y.view(torch.int16))
+    xq, sx, wq, sw, b = case
+    if k % 16 == 0:
+        odd = torch.empty(m, n + 1, dtype=torch.bfloat16, device="cuda")
+        ops.fp8_gemm(xq.cuda(), sx.cuda(), wq.cuda(), sw.cuda(), b.cuda(), out=odd[:, 1:])
+        assert torch.equal(odd[:, 1:].cpu().contiguous().view(torch.int16), y.view(torch.int16))
+    rows = torch.tensor([0, 127, 128, 255, 256, m - 1])
+    ref = S.linear_dequant_matmul(xq[rows], sx[rows], wq, sw, b)
+    assert S.max_rel_err(y[rows], ref) <= PARITY
