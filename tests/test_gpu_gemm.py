@@ -241,3 +241,19 @@ def test_auto_between_decode_and_prefill_agrees_with_every_kernel(ops, m, n, k):
     rows = torch.tensor([0, 127, 128, 255, 256, m - 1])
     ref = S.linear_dequant_matmul(xq[rows], sx[rows], wq, sw, b)
     assert S.max_rel_err(y[rows], ref) <= PARITY
+
+
+@pytest.mark.parametrize("algo", ["ALGO_TOKEN_LANE_128", "ALGO_TOKEN_LANE_256", "ALGO_TOKEN_PAIR"])
+def test_tile_after_one_that_ends_at_n_keeps_its_staging_buffers_apart(ops, algo):
+    """N = 1320 leaves 40 columns to the last tile: three stores of 16, so the CTA's next tile starts with the other staging
+    buffer.  4352 rows are more than one rasterisation group, so such tiles come in the middle of a CTA's sequence, and
+    K = 64 leaves a single K-tile between the last store and the next tile's first."""
+    m, n, k = 4352, 1320, 64
+    case = make_case(m, n, k, seed=9, bias=True)
+    xq, sx, wq, sw, b = case
+    odd = torch.empty(m, n + 1, dtype=torch.bfloat16, device="cuda")          # this row stride is stored from registers
+    ops.fp8_gemm(xq.cuda(), sx.cuda(), wq.cuda(), sw.cuda(), b.cuda(), out=odd[:, 1:], algo=getattr(ops, algo))
+    want = odd[:, 1:].cpu().contiguous()
+    assert S.max_rel_err(want, S.linear_dequant_matmul(*case)) <= PARITY
+    for _ in range(5):
+        assert torch.equal(run_gemm(ops, case, getattr(ops, algo)).view(torch.int16), want.view(torch.int16))
