@@ -73,3 +73,86 @@ def test_row_reduce_poll_gives_up_and_reports(lib):
     assert S.max_rel_err(yy.cpu(), S.linear_dequant_matmul(xq, sx, wq, sw)) <= 2e-2
     assert _cabi.device_status()["code"] == 0
     ops.check_device_status()
+
+
+class AbsentPeer:
+    """A reduction of two ranks whose second member does not exist: it occupies the stream for as long as its wait limit."""
+
+    def __init__(self, lib):
+        from nano_qwen_b200 import _cabi
+        self.lib, self.slot, self.ptrs = lib, 4096, []
+        for nbytes in (16 * self.slot, 16 * self.slot, 256):
+            p = ctypes.c_void_p()
+            _cabi.check(lib.nq_p2p_alloc(nbytes, ctypes.byref(p)), "nq_p2p_alloc")
+            self.ptrs.append(p)
+        self.inbox = (ctypes.c_void_p * 2)(self.ptrs[0].value, self.ptrs[1].value)
+        self.y = torch.ones(1024, dtype=torch.bfloat16, device="cuda")
+
+    def occupy_stream(self, ms: float):
+        assert self.lib.nq_set_wait_limit_ns(int(ms * 1e6)) == 0
+        assert self.lib.nq_row_reduce_p2p(self.y.data_ptr(), self.y.data_ptr(), self.y.numel(), self.inbox, 0, 2, self.slot,
+                                          self.ptrs[2], torch.cuda.current_stream().cuda_stream) == 0
+
+    def free(self):
+        self.lib.nq_set_wait_limit_ns(2_000_000_000)
+        torch.cuda.synchronize()
+        for p in self.ptrs:
+            self.lib.nq_p2p_free(p)
+
+
+@pytest.fixture
+def absent_peer(lib):
+    from nano_qwen_b200 import _cabi
+    torch.cuda.synchronize()
+    _cabi.device_status(reset=True)
+    peer = AbsentPeer(lib)
+    yield peer
+    peer.free()
+    _cabi.device_status(reset=True)
+
+
+def quantised(m, n, k, seed):
+    from oracle import fp8_spec as S
+    g = torch.Generator().manual_seed(seed)
+    x = torch.randn(m, k, generator=g).to(torch.bfloat16)
+    w = (torch.randn(n, k, generator=g) * 0.02).to(torch.bfloat16)
+    return x, S.quantize_act_group128(x), S.quantize_weight_block128(w)
+
+
+def decode_gemm_behind_a_waiting_reduction(lib, peer, case, algo, split_k):
+    """The GEMM starts beside the reduction, 60 ms long, and requests its weights; its activations may be read when the
+    reduction has ended, but its issuing and epilogue threads wait 2 ms only.  Returns y (a sentinel where nothing was
+    stored) and the time that the two launches took."""
+    from nano_qwen_b200 import ops
+    x, (xq, sx), (wq, sw) = case
+    x, xq, sx, wq, sw = x.cuda(), xq.cuda(), sx.t().contiguous().cuda().t(), wq.cuda(), sw.cuda()
+    y = torch.full((x.shape[0], wq.shape[0]), -777.0, dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+    t0 = time.perf_counter()
+    peer.occupy_stream(60)
+    assert lib.nq_set_wait_limit_ns(2_000_000) == 0
+    if algo == ops.ALGO_WEIGHT_LANE_FUSED:
+        ops.fp8_linear(x, wq, sw, out=y, algo=algo, split_k=split_k)
+    else:
+        ops.fp8_gemm(xq, sx, wq, sw, out=y, algo=algo, split_k=split_k)
+    lib.nq_set_wait_limit_ns(2_000_000_000)
+    torch.cuda.synchronize()
+    return y.cpu(), time.perf_counter() - t0
+
+
+@pytest.mark.parametrize("m,split_k", [(8, 8), (8, 1), (24, 4), (64, 8), (100, 8), (200, 8)])
+def test_decode_gemm_gives_up_with_copies_still_to_come(lib, absent_peer, m, split_k):
+    """With 8 splits a CTA's whole K range fits its ring: the producer never waits for a stage, it requests the activations
+    after the other roles have given up, and the CTA must not end before they have landed.  The same call then passes."""
+    from nano_qwen_b200 import _cabi, ops
+    from oracle import fp8_spec as S
+    case = quantised(m, 512, 4096, m + split_k)
+    y, waited = decode_gemm_behind_a_waiting_reduction(lib, absent_peer, case, ops.ALGO_WEIGHT_LANE, split_k)
+    status = _cabi.device_status(reset=True)
+    assert status["code"] == NQ_ERR_DEVICE_TIMEOUT
+    assert bool((y == -777.0).all()) and waited < 1.0               # every CTA gave up
+    x, (xq, sx), (wq, sw) = case
+    y = ops.fp8_gemm(xq.cuda(), sx.cuda(), wq.cuda(), sw.cuda(), algo=ops.ALGO_WEIGHT_LANE, split_k=split_k)
+    torch.cuda.synchronize()
+    assert S.max_rel_err(y.cpu(), S.linear_dequant_matmul(xq, sx, wq, sw)) <= 2e-2
+    assert _cabi.device_status()["code"] == 0
