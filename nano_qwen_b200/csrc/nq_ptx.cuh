@@ -91,7 +91,8 @@ static __device__ __noinline__ void report_timeout(DeviceStatus* status, int whe
 // role of the CTA has given up (the abort flag in shared memory).  It never branches in the calling code: after a
 // give-up `limit` is 0 and every further wait of the thread falls through at once, so the role's loop runs to its end
 // on whatever the buffers hold - its UMMAs, loads and stores stay inside the same buffers - and the kernel ends by its
-// common teardown.  Only a TMA producer has to look at gave_up() (it must not leave copies in flight behind).
+// common teardown.  A role that announces something by its own arrivals (producers of operands and of scales) has to look
+// at gave_up() and leave: an arrival on a phase that has had all of its arrivals is undefined.
 // All control flow is inside the asm statement on purpose: a C++ loop with a give-up branch around the same
 // instructions costs the UMMA issuing thread about 220 cycles per K-tile (128 x 128 x 128: 498 cycles instead of 277),
 // more than the tensor core's two queued UMMAs can hide.
