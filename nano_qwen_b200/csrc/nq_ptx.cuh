@@ -88,13 +88,14 @@ static __device__ __noinline__ void report_timeout(DeviceStatus* status, int whe
 // Bounded waits of one role of a CTA.
 //
 // wait() returns when the phase with the given parity is complete, or when it has waited for the limit, or when another
-// role of the CTA has given up (the abort flag in shared memory).  It never branches in the calling code: after a
-// give-up `limit` is 0 and every further wait of the thread falls through at once, so the role's loop runs to its end
-// on whatever the buffers hold - its UMMAs, loads and stores stay inside the same buffers - and the kernel ends by its
-// common teardown.  A role that announces something by its own arrivals (producers of operands and of scales) has to look
-// at gave_up() and leave: an arrival on a phase that has had all of its arrivals is undefined.
-// All control flow is inside the asm statement on purpose: a C++ loop with a give-up branch around the same
-// instructions costs the UMMA issuing thread about 220 cycles per K-tile (128 x 128 x 128: 498 cycles instead of 277),
+// role of the CTA has given up (the abort flag in shared memory).  After a give-up `limit` is 0 and a further wait of the
+// thread ends after two probes of its barrier (8 us on an incomplete phase).  Every role looks at gave_up():
+//   - one that announces something (producers, scale loaders, UMMA issuers of persistent kernels) leaves right after the
+//     wait, before it loads, issues or arrives: an arrival on a phase that has had all of its arrivals is undefined, and
+//     what is not announced cannot be taken for data by a role that has not given up;
+//   - an epilogue warp runs to the end of its tile on whatever the buffers hold and leaves before it stores anything.
+// The loop over the probes is inside the asm statement on purpose: as a C++ loop with the give-up inside, around the same
+// instructions, it costs the UMMA issuing thread about 220 cycles per K-tile (128 x 128 x 128: 498 cycles instead of 277),
 // more than the tensor core's two queued UMMAs can hide.
 // The limit is checked against the SM cycle counter (cheap to read; 2 cycles per nanosecond is a generous conversion).
 struct WaitCtl {

@@ -159,3 +159,37 @@ def test_decode_gemm_gives_up_with_copies_still_to_come(lib, absent_peer, algo, 
     torch.cuda.synchronize()
     assert S.max_rel_err(y.cpu(), S.linear_dequant_matmul(xq, sx, wq, sw)) <= 2e-2
     assert _cabi.device_status()["code"] == 0
+
+
+@pytest.mark.parametrize("algo", ["TOKEN_LANE_128", "TOKEN_LANE_192", "TOKEN_LANE_256", "TOKEN_PAIR"])
+@pytest.mark.parametrize("k", [128, 384])
+def test_persistent_gemm_gives_up_and_stores_no_wrong_value(lib, algo, k):
+    """Rows of y with an odd stride are stored element by element: 20 to 45 us for a tile, in which the other roles wait for
+    accumulators, stages and scale blocks.  A limit of 1 ns lets each wait probe its barrier twice (8 us), so they give up.
+    The launch ends with the status of a timeout; an element of y has its value or was left alone."""
+    from nano_qwen_b200 import _cabi, ops
+    torch.cuda.synchronize()
+    _cabi.device_status(reset=True)
+    m, n, which = 4096, 4096, getattr(ops, "ALGO_" + algo)
+    gen = torch.Generator(device="cuda").manual_seed(k)
+    xq, sx = ops.act_quant(torch.randn(m, k, generator=gen, device="cuda").to(torch.bfloat16))
+    wq, sw = ops.weight_quant(torch.randn(n, k, generator=gen, device="cuda").to(torch.bfloat16))
+    wide = torch.full((m, n + 1), -777.0, dtype=torch.bfloat16, device="cuda")
+    want = ops.fp8_gemm(xq, sx, wq, sw, algo=which)
+    torch.cuda.synchronize()
+    assert _cabi.device_status()["code"] == 0
+    try:
+        assert lib.nq_set_wait_limit_ns(1) == 0
+        t0 = time.perf_counter()
+        ops.fp8_gemm(xq, sx, wq, sw, out=wide[:, 1:], algo=which)
+        torch.cuda.synchronize()
+        waited = time.perf_counter() - t0
+    finally:
+        lib.nq_set_wait_limit_ns(2_000_000_000)
+    status = _cabi.device_status(reset=True)
+    assert status["code"] == NQ_ERR_DEVICE_TIMEOUT and waited < 0.5
+    left = wide[:, 1:] == -777.0
+    assert bool(left.any()) and bool((left | (wide[:, 1:] == want)).all()) and bool((wide[:, 0] == -777.0).all())
+    ops.fp8_gemm(xq, sx, wq, sw, out=wide[:, 1:], algo=which)
+    torch.cuda.synchronize()
+    assert torch.equal(wide[:, 1:], want) and _cabi.device_status()["code"] == 0
