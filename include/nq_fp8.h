@@ -235,8 +235,8 @@ int nq_row_reduce_pull(void* const* bufs, void* y, int64_t count, void* const* p
 
 /* Reads the device-side status block of the current device (mapped host
  * memory; call after synchronising the stream).  code = 0 or
- * NQ_ERR_DEVICE_TIMEOUT, where/block/aux say which wait expired.  `reset`
- * non-zero clears it. */
+ * NQ_ERR_DEVICE_TIMEOUT, where/block/aux say which wait expired (GEMM: aux is
+ * the K-tile).  `reset` non-zero clears it. */
 int nq_device_status(int* code, int* where, int* block, int* aux, int reset);
 
 /* Wall-clock limit (nanoseconds) of one device-side wait; default 2e9. */

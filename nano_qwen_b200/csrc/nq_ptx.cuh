@@ -20,7 +20,7 @@ struct DeviceStatus {
   int code;        // 0 = OK, else an NQ_ERR_* value written by the first failing CTA
   int where;       // site id of the wait that expired
   int block;       // blockIdx.x of the reporter
-  int aux;         // site-specific (GEMM: blockIdx.y; reductions: the peer)
+  int aux;         // site-specific (GEMM: the K-tile, for the persistent kernels' epilogue the first of its four; reductions: the peer)
 };
 
 constexpr int kErrDeviceTimeout = -5;  // mirrors NQ_ERR_DEVICE_TIMEOUT in include/nq_fp8.h
@@ -74,12 +74,12 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 
-static __device__ __noinline__ void report_timeout(DeviceStatus* status, int where) {
+static __device__ __noinline__ void report_timeout(DeviceStatus* status, int where, int aux) {
   if (status != nullptr) {
     if (atomicCAS(&status->code, 0, kErrDeviceTimeout) == 0) {
       status->where = where;
       status->block = static_cast<int>(blockIdx.x);
-      status->aux = static_cast<int>(blockIdx.y);
+      status->aux = aux;
       __threadfence_system();
     }
   }
@@ -100,25 +100,25 @@ static __device__ __noinline__ void report_timeout(DeviceStatus* status, int whe
 // The limit is checked against the SM cycle counter (cheap to read; 2 cycles per nanosecond is a generous conversion).
 struct WaitCtl {
   uint32_t limit;      // units of 1024 cycles; 0 after a give-up
-  uint32_t flag;       // shared-memory address of the CTA's abort flag
-  uint32_t site;       // wait site of this thread's first expired wait (0: none)
+  uint32_t flag;       // shared-memory address of the CTA's abort flag: 0, or site + 256 * tile of an expired wait
 
-  __device__ __forceinline__ WaitCtl(int* abort_flag, uint64_t limit_ns) : flag(smem_u32(abort_flag)), site(0) {
+  __device__ __forceinline__ WaitCtl(int* abort_flag, uint64_t limit_ns) : flag(smem_u32(abort_flag)) {
     const uint64_t units = (limit_ns >> 9) + 1;
     limit = units < 0x7FFFFFFFull ? static_cast<uint32_t>(units) : 0x7FFFFFFFu;
   }
 
+  // `tile`: what to report with the site
   template <int SITE>
-  __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity) {
+  __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity, int tile) {
     asm volatile(
         "{\n\t.reg .pred P;\n\t.reg .u64 t0, t1;\n\t.reg .u32 f;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 P, [%2], %3;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
         "@P bra DONE;\n\t"
         "mov.u64 t0, %%clock64;\n\t"
         "AGAIN:\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 P, [%2], %3;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
         "@P bra DONE;\n\t"
-        "ld.volatile.shared.u32 f, [%4];\n\t"
+        "ld.volatile.shared.u32 f, [%3];\n\t"
         "setp.ne.u32 P, f, 0;\n\t"
         "@P bra STOP;\n\t"
         "mov.u64 t1, %%clock64;\n\t"
@@ -127,21 +127,32 @@ struct WaitCtl {
         "cvt.u32.u64 f, t1;\n\t"
         "setp.lt.u32 P, f, %0;\n\t"
         "@P bra AGAIN;\n\t"
-        "mov.u32 %1, %5;\n\t"
-        "mov.u32 f, 1;\n\t"
-        "st.volatile.shared.u32 [%4], f;\n\t"
+        "shl.b32 f, %5, 8;\n\t"
+        "add.u32 f, f, %4;\n\t"
+        "st.volatile.shared.u32 [%3], f;\n\t"
         "STOP:\n\t"
         "mov.u32 %0, 0;\n\t"
         "DONE:\n\t}"
-        : "+r"(limit), "+r"(site)
-        : "r"(bar), "r"(parity), "r"(flag), "n"(SITE)
+        : "+r"(limit)
+        : "r"(bar), "r"(parity), "r"(flag), "n"(SITE), "r"(tile)
         : "memory");
   }
   template <int SITE>
-  __device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity) { wait<SITE>(smem_u32(bar), parity); }
+  __device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity, int tile) { wait<SITE>(smem_u32(bar), parity, tile); }
   __device__ __forceinline__ bool gave_up() const { return limit == 0; }
-  __device__ __forceinline__ void report(DeviceStatus* status) const {
-    if (site != 0) report_timeout(status, static_cast<int>(site));
+  // The first to get here reports the wait that expired: a role when it leaves (a kernel that is stuck behind another one
+  // says so at once), or for the epilogue the CTA's teardown.  k_tile(site, tile) makes a K-tile of what wait() was given.
+  template <typename F>
+  static __device__ __forceinline__ void report_flag(int flag, DeviceStatus* status, F k_tile) {
+    report_timeout(status, flag & 255, k_tile(flag & 255, flag >> 8));
+  }
+  template <typename F>
+  __device__ __forceinline__ void report(DeviceStatus* status, F k_tile) const {
+    if (gave_up()) {
+      int f;
+      asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(f) : "r"(flag) : "memory");
+      report_flag(f, status, k_tile);
+    }
   }
 };
 

@@ -16,6 +16,8 @@ pytestmark = pytest.mark.gpu
 
 NQ_ERR_DEVICE_TIMEOUT = -5
 SITE_ROW_REDUCE = 64
+SITE_PRODUCER, SITE_MMA_FULL, SITE_MMA_TMEM_EMPTY, SITE_EPI_TMEM_FULL, SITE_SCALE_FULL, SITE_SCALE_EMPTY = 1, 2, 3, 4, 5, 6
+SITE_WEIGHT_LANE = 16
 
 
 @pytest.fixture(scope="module")
@@ -153,6 +155,12 @@ def test_decode_gemm_gives_up_with_copies_still_to_come(lib, absent_peer, algo, 
     y, waited = decode_gemm_behind_a_waiting_reduction(lib, absent_peer, case, getattr(ops, "ALGO_" + algo), split_k)
     status = _cabi.device_status(reset=True)
     assert status["code"] == NQ_ERR_DEVICE_TIMEOUT
+    # the issuer's or the epilogue's first wait, at once (the reduction's own limit expires 58 ms later); the fused kernel's
+    # producer waits for nothing else than its first stage, to which it comes back after the fifth K-tile
+    first = [(4096 // 128) * z // split_k for z in range(split_k)]
+    expired = (status["where"] - SITE_WEIGHT_LANE, status["aux"])
+    assert expired[0] in (SITE_MMA_FULL, SITE_EPI_TMEM_FULL) and expired[1] in first or (
+        algo == "WEIGHT_LANE_FUSED" and expired[0] == SITE_PRODUCER and expired[1] - 5 in first), expired
     assert bool((y == -777.0).all()) and waited < 1.0               # every CTA gave up
     x, (xq, sx), (wq, sw) = case
     y = ops.fp8_gemm(xq.cuda(), sx.cuda(), wq.cuda(), sw.cuda(), algo=ops.ALGO_WEIGHT_LANE, split_k=split_k)
@@ -188,6 +196,8 @@ def test_persistent_gemm_gives_up_and_stores_no_wrong_value(lib, algo, k):
         lib.nq_set_wait_limit_ns(2_000_000_000)
     status = _cabi.device_status(reset=True)
     assert status["code"] == NQ_ERR_DEVICE_TIMEOUT and waited < 0.5
+    assert status["where"] in (SITE_PRODUCER, SITE_MMA_FULL, SITE_MMA_TMEM_EMPTY, SITE_EPI_TMEM_FULL, SITE_SCALE_FULL, SITE_SCALE_EMPTY)
+    assert 0 <= status["aux"] < k // 128 and 0 <= status["block"] < 148
     left = wide[:, 1:] == -777.0
     assert bool(left.any()) and bool((left | (wide[:, 1:] == want)).all()) and bool((wide[:, 0] == -777.0).all())
     ops.fp8_gemm(xq, sx, wq, sw, out=wide[:, 1:], algo=which)
