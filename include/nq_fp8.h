@@ -247,6 +247,10 @@ int nq_set_wait_limit_ns(uint64_t ns);
  * read at launch time.  Returns the previous value, or a negative status for n < 0. */
 int nq_set_sm_reserve(int n);
 
+/* The NQ_ALGO_* that NQ_ALGO_AUTO stands for with these sizes on a GPU of `sm_count` SMs, under the present
+ * nq_set_sm_reserve: NQ_ALGO_WEIGHT_LANE, NQ_ALGO_TOKEN_LANE_128, _256 or NQ_ALGO_TOKEN_PAIR.  Host only, needs no GPU. */
+int nq_gemm_auto_algo(int64_t M, int64_t N, int split_k, int sm_count);
+
 /* Number of kernels this library has launched on the calling process so far. */
 int64_t nq_launch_count(void);
 

@@ -53,6 +53,7 @@ SIGNATURES = {
     "nq_device_status": (c_int, [POINTER(c_int), POINTER(c_int), POINTER(c_int), POINTER(c_int), c_int]),
     "nq_set_wait_limit_ns": (c_int, [c_uint64]),
     "nq_set_sm_reserve": (c_int, [c_int]),
+    "nq_gemm_auto_algo": (c_int, [c_int64, c_int64, c_int, c_int]),
     "nq_launch_count": (c_int64, []),
 }
 

@@ -154,6 +154,22 @@ int validate_gemm(const GemmArgs& a) {
   return NQ_OK;
 }
 
+// What NQ_ALGO_AUTO launches.
+int auto_algo(int64_t M, int64_t N, int split_k, int sm_count) {
+  // Measured crossover on B200 (CUDA graph, 8B layer shapes): weight rows on the lanes up to 64 tokens; at 72 tokens the
+  // token-lane kernel is ahead (65 us against 73 us for the four linears of a layer).
+  if (M <= 64) return NQ_ALGO_WEIGHT_LANE;
+  // Prefill-sized launches with at least two rounds of 256 x 256 tiles go to the CTA-pair kernel: alone it runs
+  // level with the single-CTA kernel (2.0-2.1 PFLOP/s), inside a long power-capped step it is 1-2 % ahead
+  // (a third fewer operand bytes cross the L2 -> SM path; three interleaved runs of the 36-layer step each).
+  // (No kernel splits K in launches of that many tiles: a caller's split_k has no effect there.)
+  if (M >= 2048 && ((M + 255) / 256) * ((N + 255) / 256) >= 2 * persistent_pairs(sm_count)) return NQ_ALGO_TOKEN_PAIR;
+  // In between, rounds of tiles decide (pick_token_tile): the four linears of an 8B layer take 171 us against 180 with
+  // the pair kernel left out (520 tokens), 204 / 208 (777), 217 / 228 (1024), 309 / 321 (1536).  A caller's K split goes
+  // to the kernels that can split.
+  return pick_token_tile(M, N, sm_count, split_k <= 1);
+}
+
 int gemm_dispatch(const GemmArgs& a, int algo) {
   int st = validate_gemm(a);
   if (st != NQ_OK) return st;
@@ -161,25 +177,13 @@ int gemm_dispatch(const GemmArgs& a, int algo) {
   DeviceCtx* ctx = nullptr;
   st = ensure_init(&ctx);
   if (st != NQ_OK) return st;
-  // Measured crossover on B200 (CUDA graph, 8B layer shapes): weight rows on the lanes up to 64 tokens; at 72 tokens the
-  // token-lane kernel is ahead (65 us against 73 us for the four linears of a layer).
-  // Prefill-sized launches with at least two rounds of 256 x 256 tiles go to the CTA-pair kernel: alone it runs
-  // level with the single-CTA kernel (2.0-2.1 PFLOP/s), inside a long power-capped step it is 1-2 % ahead
-  // (a third fewer operand bytes cross the L2 -> SM path; three interleaved runs of the 36-layer step each).
-  // In between, rounds of tiles decide (pick_token_tile): the four linears of an 8B layer take 171 us against 180 with
-  // the pair kernel left out (520 tokens), 204 / 208 (777), 217 / 228 (1024), 309 / 321 (1536).  A caller's K split goes
-  // to the kernels that can split.
-  if (algo == NQ_ALGO_AUTO) {
-    if (a.M <= 64) algo = NQ_ALGO_WEIGHT_LANE;
-    else if (a.M >= 2048 && ((a.M + 255) / 256) * ((a.N + 255) / 256) >= ctx->sm_count) algo = NQ_ALGO_TOKEN_PAIR;
-    else algo = pick_token_tile(a.M, a.N, ctx->sm_count, a.split_k <= 1) == TokenTile::kPair ? NQ_ALGO_TOKEN_PAIR : NQ_ALGO_TOKEN_LANE;
-  }
+  if (algo == NQ_ALGO_AUTO) algo = auto_algo(a.M, a.N, a.split_k, ctx->sm_count);
   if (algo == NQ_ALGO_TOKEN_LANE) return launch_gemm_token_lane(a, ctx, 0);
   if (algo == NQ_ALGO_TOKEN_LANE_128) return launch_gemm_token_lane(a, ctx, 128);
   if (algo == NQ_ALGO_TOKEN_LANE_192) return launch_gemm_token_lane(a, ctx, 192);
   if (algo == NQ_ALGO_TOKEN_LANE_256) return launch_gemm_token_lane(a, ctx, 256);
   if (algo == NQ_ALGO_WEIGHT_LANE) return launch_gemm_weight_lane(a, ctx);
-  if (algo == NQ_ALGO_TOKEN_PAIR) return launch_gemm_token_pair(a, ctx, 256);
+  if (algo == NQ_ALGO_TOKEN_PAIR) return launch_gemm_token_pair(a, ctx);
   return NQ_ERR_BAD_ARGUMENT;
 }
 
@@ -317,6 +321,11 @@ int nq_set_wait_limit_ns(uint64_t ns) {
 int nq_set_sm_reserve(int n) {
   if (n < 0) return NQ_ERR_BAD_ARGUMENT;
   return g_sm_reserve.exchange(n);
+}
+
+int nq_gemm_auto_algo(int64_t M, int64_t N, int split_k, int sm_count) {
+  if (M < 1 || N < 1 || sm_count < 2) return NQ_ERR_BAD_ARGUMENT;
+  return auto_algo(M, N, split_k, sm_count);
 }
 
 int64_t nq_launch_count(void) { return g_launches.load(); }

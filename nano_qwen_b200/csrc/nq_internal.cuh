@@ -47,11 +47,19 @@ struct GemmArgs {
   cudaStream_t stream;
   bool pdl;
 };
-enum class TokenTile { k128, k256, kPair };
-TokenTile pick_token_tile(int64_t M, int64_t N, int sm_count, bool pairs);   // which kernel, for more than 64 tokens
+// CTAs and CTA pairs of the persistent kernels: one per SM, less the SMs held back (nq_set_sm_reserve).
+inline int persistent_ctas(int sm_count) {
+  const int n = sm_count - sm_reserve();
+  return n < sm_count / 2 ? sm_count / 2 : n;
+}
+inline int persistent_pairs(int sm_count) {
+  const int n = (sm_count - sm_reserve()) / 2;
+  return n < 1 ? 1 : n;
+}
+int pick_token_tile(int64_t M, int64_t N, int sm_count, bool pairs);   // for more than 64 tokens: the NQ_ALGO_TOKEN_* to launch
 int launch_gemm_token_lane(const GemmArgs& a, DeviceCtx* ctx, int tile_n);   // tile_n: 0 = choose, else 128/192/256
 int launch_gemm_weight_lane(const GemmArgs& a, DeviceCtx* ctx);
-int launch_gemm_token_pair(const GemmArgs& a, DeviceCtx* ctx, int tile_n);   // 256 x tile_n tiles on CTA pairs (cta_group::2)
+int launch_gemm_token_pair(const GemmArgs& a, DeviceCtx* ctx);   // 256 x 256 tiles on CTA pairs (cta_group::2)
 size_t weight_lane_workspace_bytes(int64_t M, int64_t N, int64_t K);
 int weight_lane_pick_split(int64_t M, int64_t N, int64_t K, int sm_count);
 int setup_gemm_kernels();   // cudaFuncSetAttribute for the large dynamic shared memory

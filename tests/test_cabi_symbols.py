@@ -34,6 +34,40 @@ def test_version_and_status_strings(built_library):
     assert lib.nq_launch_count() >= 0
 
 
+def test_auto_dispatch_by_rounds_of_tiles(built_library):
+    """Both sides of each line of the rule, with 148 SMs: the choice needs no GPU."""
+    from nano_qwen_b200 import _cabi
+    lib = _cabi.lib()
+    W, T128, T256, PAIR = _cabi.ALGO_WEIGHT_LANE, _cabi.ALGO_TOKEN_LANE_128, _cabi.ALGO_TOKEN_LANE_256, _cabi.ALGO_TOKEN_PAIR
+    for m, n, split, want in [
+            (1, 4096, 0, W), (64, 24576, 0, W), (65, 24576, 0, T256),         # 192 tiles of 128 x 128 and 96 of 128 x 256
+            (128, 148 * 128, 0, T128), (128, 149 * 128, 0, T256),             # one round of 128-wide tiles, and one tile more
+            (4096, 128, 0, T128), (4096, 129, 0, T128),
+            (520, 4104, 0, PAIR), (520, 4104, 1, PAIR), (520, 4104, 2, T256), # a K split goes to a kernel that can split
+            (777, 6144, 0, T128), (777, 24576, 0, T256), (1281, 4088, 0, T128), (2047, 1000, 0, T128),
+            (2047, 4736, 0, T128), (2048, 4736, 0, PAIR), (2048, 4736, 4, PAIR), (8192, 6144, 0, PAIR)]:
+        assert lib.nq_gemm_auto_algo(m, n, split, 148) == want, (m, n, split)
+    assert lib.nq_gemm_auto_algo(0, 128, 0, 148) == lib.nq_gemm_auto_algo(1, 128, 0, 0) == -1
+
+
+def test_auto_dispatch_counts_rounds_without_the_sms_held_back(built_library):
+    """140 tiles of 128 x 128 are one round of 148 SMs and two of 128, where 70 tiles of 128 x 256 are one."""
+    from nano_qwen_b200 import _cabi
+    lib = _cabi.lib()
+    old = lib.nq_set_sm_reserve(0)
+    try:
+        assert lib.nq_gemm_auto_algo(512, 35 * 128, 2, 148) == _cabi.ALGO_TOKEN_LANE_128
+        assert lib.nq_gemm_auto_algo(2048, 34 * 128, 0, 148) == _cabi.ALGO_TOKEN_PAIR            # 8 x 17 tiles: two rounds
+        lib.nq_set_sm_reserve(20)
+        assert lib.nq_gemm_auto_algo(512, 35 * 128, 2, 148) == _cabi.ALGO_TOKEN_LANE_256
+        assert lib.nq_gemm_auto_algo(2048, 34 * 128, 0, 148) == _cabi.ALGO_TOKEN_PAIR
+        lib.nq_set_sm_reserve(1000)                                           # at least half of the SMs stay
+        assert lib.nq_gemm_auto_algo(512, 18 * 128, 2, 148) == _cabi.ALGO_TOKEN_LANE_128         # 72 tiles, 74 CTAs
+        assert lib.nq_gemm_auto_algo(512, 19 * 128, 2, 148) == _cabi.ALGO_TOKEN_LANE_256
+    finally:
+        lib.nq_set_sm_reserve(old)
+
+
 def test_no_cpu_fallback():
     """Without a CUDA device every compute entry refuses loudly instead of computing elsewhere."""
     import pytest

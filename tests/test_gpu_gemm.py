@@ -227,7 +227,7 @@ def test_status_block_clean_after_all_gemms(ops):
     (2047, 1000, 200),
 ])
 def test_auto_between_decode_and_prefill_agrees_with_every_kernel(ops, m, n, k):
-    """The rule by rounds of tiles sends these to different kernels; unsplit, all of them add the K-tiles in one order, so
+    """The rule by rounds of tiles (tests/test_cabi_symbols.py) sends these to different kernels; unsplit, all of them add the K-tiles in one order, so
     the bits agree, and rows whose stride allows no bulk stores take the same route."""
     case = make_case(m, n, k, seed=m + n, bias=True)
     y = run_gemm(ops, case, ops.ALGO_AUTO, split_k=1)
