@@ -134,6 +134,7 @@ __global__ void __launch_bounds__(256, 6) silu_mul_quant_kernel(const __nv_bfloa
 // Two passes over the row by 256 threads took 2.8 us at 4096 columns and 4.1 us at 5120 (whose last 1024 columns were a
 // second trip of a quarter of the threads); now 2.2 and 2.4 us.  Large batches are bound by HBM (7 bytes per element):
 // a CTA requests its next row before it reduces the present one; 8192 rows of 4096: 54 -> 50 us (36 us at copy rate).
+// Without a residual a thread has half the bytes in flight, and many long rows go to the two-pass kernel (two_pass_norm).
 __global__ void __launch_bounds__(1024, 1) rmsnorm_row_quant_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* res_in,
                                                                     const __nv_bfloat16* __restrict__ weight, float eps, int gemma,
                                                                     int64_t M, int64_t H, int64_t ldx, int64_t ld_res,
@@ -224,9 +225,11 @@ __global__ void __launch_bounds__(1024, 1) rmsnorm_row_quant_kernel(const __nv_b
   }
 }
 
-// Rows of more than 8192 elements.  One CTA of 256 threads per token row.  Pass 1: x (+ residual) in fp32, sum of squares.  Pass 2 reads the row again
-// (from L1/L2), writes the new residual, normalises, rounds to bf16, multiplies by the weight in bf16 and quantises.
-// (Keeping the row in registers between the passes was measured slower: 80 registers halve the CTAs per SM.)
+// Rows of more than 8192 elements, and large batches of long rows (two_pass_norm).  One CTA of 256 threads per token row.
+// Pass 1: x (+ residual) in fp32, sum of squares.  Pass 2 reads the row again (from L1/L2), writes the new residual,
+// normalises, rounds to bf16, multiplies by the weight in bf16 and quantises.  Eight rows of 48 registers per SM keep more
+// bytes in flight than the row kernel's one or two where all of them matter: 8192 rows of 5120 without a residual 53 us
+// against 69.  (Keeping the row in registers between these passes was slower: 80 registers halve the CTAs per SM.)
 __global__ void __launch_bounds__(256) rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* res_in,
                                                             const __nv_bfloat16* __restrict__ weight, float eps, int gemma,
                                                             int64_t H, int64_t ldx, int64_t ld_res, __nv_bfloat16* res_out,
@@ -317,6 +320,22 @@ __global__ void __launch_bounds__(256) rmsnorm_quant_kernel(const __nv_bfloat16*
   }
 }
 
+// Which of the two norm kernels; their sums have the same order and their results the same bits.  Measured, two-pass against
+// row kernel, us.  Without a residual: 3072 columns 10.6 / 10.5 (2048 rows), 14.2 / 14.5 (3001), 34 / 37 (8192); 4096 columns
+// 6.4 / 6.4 (777), 7.6 / 8.0 (1024), 38 / 46 (8192); 4352 columns (a second trip for a few lanes) 10.9 / 9.9 (1024),
+// 11.8 / 12.2 (1280); 5120 columns 6.9 / 6.5 (512), 7.0 / 7.6 (640), 9.4 / 8.9 (777), 10.3 / 10.1 (1024), 11.4 / 12.7 (1280),
+// 53 / 69 (8192); 8192 columns 8.7 / 8.3 (512), 9.1 / 9.9 (640), 10.7 / 11.6 (777), 67 / 90 (8192).
+// With one: 7168 columns 92.2 / 91.1 (8192), 174 / 177 (16384); 8192 columns 42.5 / 41.0 (3001), 98.3 / 100.9 (8192).
+bool two_pass_norm(int64_t M, int64_t H, bool residual, int sm_count) {
+  if (H > 8192) return true;
+  if (residual) return H >= 7168 && M * H >= (1 << 26);
+  if (H <= 2560) return false;
+  if (H <= 4096) return M >= (H >= 3840 ? 1024 : H >= 3328 ? 1280 : 2560);
+  // the row kernel has one CTA per SM, the two-pass kernel five: its first wave ends with the fifth round of the other
+  const int64_t rounds = (M + sm_count - 1) / sm_count;
+  return rounds == 5 || rounds >= (H < 4608 ? 9 : H < 6144 ? 7 : 6);
+}
+
 bool aligned16p(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 }  // namespace
@@ -384,7 +403,7 @@ int nq_rmsnorm_quant_e4m3_g128(const void* x, const void* residual_in, const voi
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (H <= 8192) {
+  if (!two_pass_norm(M, H, residual_in != nullptr, ctx->sm_count)) {
     const int64_t threads = (H + 255) / 256 * 32;
     // as many CTAs as are resident at once (63 registers: 1024 threads per SM); asking for 1536 threads per SM cost 5-10 %
     const int64_t slots = ctx->sm_count * (1024 / threads);

@@ -141,6 +141,59 @@ def test_rmsnorm_quant_many_rows_in_place(ops, h):
         check_quantised(xq[rows.cuda()].view(torch.float8_e4m3fn), sx[:, rows.cuda()].t(), ref)
 
 
+@pytest.mark.parametrize("h,m,with_residual", [(2576, 2560, False), (3328, 1280, False), (3840, 1024, False), (4096, 1024, False),
+                                               (4112, "8 * sm + 1", False), (4112, "5 * sm + 1", False), (4608, "6 * sm + 1", False),
+                                               (5120, "4 * sm + 1", False), (8192, "4 * sm + 1", False),
+                                               (7168, 9363, True), (8192, 8192, True), (8208, 1, True), (8208, 1, False)])
+def test_rmsnorm_quant_same_bits_on_both_sides_of_the_dispatch(ops, h, m, with_residual):
+    """With m rows one of the two kernels runs, with one row less the other (above 8192 columns always the two-pass kernel):
+    rows, scales, residual and bf16 results have the same bits, strided rows and gemma weights included."""
+    m = eval(str(m), {"sm": torch.cuda.get_device_properties(0).multi_processor_count})
+    gen = torch.Generator(device="cuda").manual_seed(h)
+    x = torch.randn(m, h + 8, generator=gen, device="cuda").to(torch.bfloat16)[:, :h]
+    res = torch.randn(m, h, generator=gen, device="cuda").to(torch.bfloat16) if with_residual else None
+    w = torch.randn(h, generator=gen, device="cuda").to(torch.bfloat16)
+    many = ops.rmsnorm_quant(x, w, 1e-6, res, gemma=True, want_bf16=True)
+    if m > 1:
+        few = ops.rmsnorm_quant(x[:m - 1], w, 1e-6, None if res is None else res[:m - 1], gemma=True, want_bf16=True)
+        for a, b in zip(many, few):
+            assert (a is None) == (b is None)
+            if a is not None:
+                a, b = a[:m - 1].contiguous(), b.contiguous()
+                assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+    rows = torch.tensor([0, m // 2, m - 1])
+    ref = R.rms_norm(x[rows.cuda()].cpu(), w.cpu(), 1e-6, None if res is None else res[rows.cuda()].cpu(), gemma=True)
+    check_bf16(many[3][rows.cuda()], ref[0] if with_residual else ref)
+
+
+@pytest.mark.parametrize("h,m", [(16, 3), (272, 3), (1024, 3), (4112, 3), (5120, 3), (8192, 3), (8208, 3), (12288, 2), (4096, 1024)])
+def test_rmsnorm_quant_order_of_the_sum(ops, h, m):
+    """The sum of squares of either kernel, in fp32: 256 strips take 16 elements each, one by one, and go on 4096 elements
+    further; 32 strips are added as a tree, the 8 trees one after the other.  Evaluated here in that order, the bf16 results
+    have the same bits (a sum in another order moves some of them)."""
+    g = torch.Generator().manual_seed(h)
+    x = torch.randn(m, h, generator=g).to(torch.bfloat16)
+    w = torch.randn(h, generator=g).to(torch.bfloat16)
+    y = ops.rmsnorm_quant(x.cuda(), w.cuda(), 1e-6, want_bf16=True)[3].cpu()
+    v = x[-3:].float().numpy()
+    padded = np.zeros((v.shape[0], -(-h // 4096) * 4096), dtype=np.float32)
+    padded[:, :h] = v
+    blocks = padded.reshape(v.shape[0], -1, 256, 16)                    # [row, trip, strip, element]
+    part = np.zeros((v.shape[0], 256), dtype=np.float32)
+    for trip in range(blocks.shape[1]):
+        for e in range(16):                                             # fma: exact square, one rounding
+            part = (blocks[:, trip, :, e].astype(np.float64) ** 2 + part).astype(np.float32)
+    part = part.reshape(v.shape[0], 8, 32)
+    for half in (16, 8, 4, 2, 1):
+        part = part[:, :, :half] + part[:, :, half:2 * half]
+    total = np.zeros(v.shape[0], dtype=np.float32)
+    for i in range(8):
+        total = total + part[:, i, 0]
+    rstd = np.float32(1.0) / np.sqrt(total / np.float32(h) + np.float32(1e-6))
+    want = torch.from_numpy(v * rstd[:, None].astype(np.float32)).to(torch.bfloat16) * w
+    assert torch.equal(y[-3:].view(torch.int16), want.view(torch.int16))
+
+
 @pytest.mark.parametrize("m", [1, 888, 889])
 def test_silu_mul_quant_narrow_and_wide_lanes(ops, m):
     """Groups of 8 elements per lane up to one wave of CTAs (148 SMs: 14208 groups = 888 rows of 16), of 16 beyond: the same
