@@ -465,10 +465,17 @@ __device__ __forceinline__ float2 bf16x2_unpack(uint32_t w) {
 // E bf16 values of one lane, as E / 2 packed pairs -> amax over the 128 / E lanes of the group -> scale -> E e4m3 bytes.
 template <int E>
 __device__ __forceinline__ void quantise_packed(const uint32_t (&h)[E / 2], uint32_t lanes, float& scale, uint32_t (&q)[E / 4]) {
-  uint32_t m2 = 0u;                                          // a maximum of bf16 values is exact
+  // A maximum of bf16 values is exact, in any order: a tree, since small batches are bound by this lane's chain (a chain of
+  // E / 2 maxima made 144 rows of 6400 2.5 us, the tree 2.3).
+  uint32_t m2[E / 4];
 #pragma unroll
-  for (int i = 0; i < E / 2; ++i) m2 = bf16x2_absmax(m2, h[i]);
-  float amax = fmaxf(bf16_bits_to_float(m2 & 0xFFFFu), bf16_bits_to_float(m2 >> 16));
+  for (int i = 0; i < E / 4; ++i) m2[i] = bf16x2_absmax(h[2 * i], h[2 * i + 1]);
+#pragma unroll
+  for (int n = E / 8; n > 0; n /= 2) {
+#pragma unroll
+    for (int i = 0; i < n; ++i) m2[i] = bf16x2_absmax(m2[i], m2[i + n]);
+  }
+  float amax = fmaxf(bf16_bits_to_float(m2[0] & 0xFFFFu), bf16_bits_to_float(m2[0] >> 16));
 #pragma unroll
   for (int o = 1; o < 128 / E; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(lanes, amax, o));
   scale = __fdiv_rn(fmaxf(amax, 1e-10f), 448.0f);
