@@ -139,7 +139,8 @@ def rmsnorm_quant(x: torch.Tensor, weight: torch.Tensor, eps: float, residual: t
             raise TypeError("residual must be bfloat16 with the shape of x")
         if residual.stride(1) != 1:
             residual = residual.contiguous()
-        res_out = torch.empty((M, H), dtype=torch.bfloat16, device=x.device)
+        # the kernel reads and writes the residual with one row stride
+        res_out = torch.empty_strided((M, H), (residual.stride(0) if M > 1 else H, 1), dtype=torch.bfloat16, device=x.device)
     y = torch.empty((M, H), dtype=torch.bfloat16, device=x.device) if want_bf16 else None
     xq, sx, ld_xq, ld_sx = _quant_buffers(M, H, x.device)
     if M > 0 and H > 0:

@@ -296,3 +296,20 @@ def test_mlp_block_with_fused_producers_matches_the_oracle_chain(built_library, 
     y_ref = lin(R.silu_and_mul(lin(h_ref, w1)), w2)
     assert torch.equal(new_res.cpu().view(torch.int16), res_ref.view(torch.int16))
     assert S.max_rel_err(y.cpu(), y_ref) <= 2e-2
+
+
+@pytest.mark.parametrize("h", [256, 8208])
+def test_rmsnorm_quant_residual_with_strided_rows(ops, h):
+    """A residual that is a column slice of a wider buffer: the new one has its row stride, nothing else is written."""
+    m, pad = 37, 24
+    gen = torch.Generator(device="cuda").manual_seed(h)
+    x = torch.randn(m, h, generator=gen, device="cuda").to(torch.bfloat16)
+    wide = torch.randn(m, h + pad, generator=gen, device="cuda").to(torch.bfloat16)
+    w = torch.randn(h, generator=gen, device="cuda").to(torch.bfloat16)
+    before = wide.clone()
+    got = ops.rmsnorm_quant(x, w, 1e-6, wide[:, 8:8 + h])
+    want = ops.rmsnorm_quant(x, w, 1e-6, wide[:, 8:8 + h].contiguous())
+    for a, b in zip(got[:3], want[:3]):
+        assert a.shape == b.shape and torch.equal(a.contiguous().view(torch.uint8), b.contiguous().view(torch.uint8))
+    assert got[2].stride() == (h + pad, 1) and torch.equal(wide, before)
+    assert torch.equal(got[2], (x.float() + wide[:, 8:8 + h].float()).to(torch.bfloat16))
