@@ -22,9 +22,16 @@ def _round_up(v: int, m: int) -> int:
     return (v + m - 1) // m * m
 
 
+# What torch's own generated code asks for the stream; not part of its public interface, so not taken for granted.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device = getattr(torch._C, "_cuda_getDevice", None)
+
+
 def _stream() -> int:
     """Handle of the current stream of the current device (without building a Stream object: 3 us a call)."""
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    if _raw_stream is None or _device is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_device())
 
 
 def _require_cuda(*tensors: torch.Tensor) -> None:

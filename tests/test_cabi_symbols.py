@@ -82,6 +82,20 @@ def test_no_cpu_fallback():
             ops.init()
 
 
+def test_stream_handle_without_torchs_private_names(monkeypatch):
+    """The raw-handle query is a shortcut: a torch without it is asked through its public interface."""
+    import types
+    from nano_qwen_b200 import ops
+    monkeypatch.setattr(ops, "_raw_stream", lambda device: 1000 + device, raising=False)
+    monkeypatch.setattr(ops, "_device", lambda: 3, raising=False)
+    assert ops._stream() == 1003
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: types.SimpleNamespace(cuda_stream=7))
+    for name in ("_raw_stream", "_device"):
+        with monkeypatch.context() as m:
+            m.setattr(ops, name, None)
+            assert ops._stream() == 7
+
+
 def test_product_never_imports_the_oracle():
     pkg = os.path.join(ROOT, "nano_qwen_b200")
     for dirpath, _, files in os.walk(pkg):
