@@ -128,8 +128,10 @@ size_t nq_fp8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K);
 /* y = bf16( sum_t sx[t,m] * sw[n/128,t] * (xq[m, tile t] . wq[n, tile t]) + bias[n] ),
  * tile = 128 consecutive k; inner products accumulate in fp32 on the tensor
  * cores, the scaled sum over tiles in fp32 registers.
- * `split_k` = 0 lets the library choose; otherwise it is a hint for
- * NQ_ALGO_WEIGHT_LANE. */
+ * `split_k` = 0 lets the library choose; otherwise it is a hint for the kernels
+ * that split K (weight-lane, and token-lane with 4 K-tiles or more to a split).
+ * After an expired wait (nq_device_status) an element of y has its value or was
+ * left alone, except where K is split: a sum over splits may then be wrong. */
 int nq_fp8_gemm_bs128(const void* xq, int64_t ld_xq, const float* sx, int64_t ld_sx,
                       const void* wq, int64_t ld_wq, const float* sw, int64_t ld_sw,
                       const void* bias, void* y, int64_t ldy,

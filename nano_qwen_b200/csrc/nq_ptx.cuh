@@ -33,7 +33,6 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-__device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
 
 // ------------------------------- mbarrier --------------------------------- //
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
@@ -213,11 +212,6 @@ __device__ __forceinline__ uint64_t l2_policy_evict_first() {
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
-__device__ __forceinline__ uint64_t l2_policy_evict_last() {
-  uint64_t p;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
 
 // Programmatic dependent launch: wait for the kernels this one depends on /
 // let the next kernel in the stream start its prologue.
@@ -307,9 +301,6 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t local_smem_addr, uint32
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t bar_cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
-}
 
 // Shared-memory matrix descriptor for a K-major operand tile whose rows are
 // exactly 128 bytes (one 128-byte swizzle atom wide), rows 8-by-8 in 1024-byte
@@ -370,8 +361,7 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
       : "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// Same wait, tied to the destination registers of a load so that the compiler cannot
+// Waits for the tensor-memory loads of the warp, tied to the destination registers of one so that the compiler cannot
 // schedule a consumer of those registers ahead of it.
 __device__ __forceinline__ void tmem_ld_wait_on(uint32_t (&r)[32]) {
   asm volatile(

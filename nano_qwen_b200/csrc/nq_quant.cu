@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(256, E == 8 ? 6 : 1) act_quant_kernel(const __
 // Bound by HBM (2 bytes in, 1 byte out per weight): the block is read once and stays in registers between the amax
 // and the division (32 per thread), a half-warp reads 256 and writes 128 consecutive bytes, and the quotient costs
 // three packed instructions per pair instead of two IEEE divisions.  Two matrices of 12288 x 4096, written straight
-// into the merged parameter: 53 us = 5.7 TB/s (two passes of 128-byte segments per thread, IEEE divisions and a copy
+// into the merged parameter: 53-57 us = 5.3-5.7 TB/s (two passes of 128-byte segments per thread, IEEE divisions and a copy
 // of the result into the parameter: 168 us).
 // VEC: 16-byte loads and 8-byte stores, possible when K and both row strides are multiples of 8 and the bases are
 // aligned; otherwise element by element.

@@ -117,7 +117,8 @@ def test_rmsnorm_quant_many_rows_in_place(ops, h):
     """More rows than CTAs (each takes several, the next one requested early), the residual updated in place, strided
     rows; 8192 columns fill a CTA, 8208 take the two-pass kernel.  Row by row equal to calls with one row each."""
     from nano_qwen_b200 import _cabi
-    m, pad = 148 * max(1, 1024 // (-(-h // 256) * 32)) + 151, 16
+    sm = torch.cuda.get_device_properties(0).multi_processor_count
+    m, pad = sm * max(1, 1024 // (-(-h // 256) * 32)) + sm + 3, 16
     gen = torch.Generator(device="cuda").manual_seed(h)
     x = torch.randn(m, h + pad, generator=gen, device="cuda").to(torch.bfloat16)
     res = torch.randn(m, h + pad, generator=gen, device="cuda").to(torch.bfloat16)
@@ -132,10 +133,10 @@ def test_rmsnorm_quant_many_rows_in_place(ops, h):
     assert st == 0
     want = torch.cat([res[:, :h].float().add(x[:, :h].float()).to(torch.bfloat16), res[:, h:]], 1)
     assert torch.equal(new.view(torch.int16), want.view(torch.int16))
-    for r in (0, 1, 147, 148, m // 2, m - 2, m - 1):
+    for r in (0, 1, sm - 1, sm, m // 2, m - 2, m - 1):
         q1, s1, _, _ = ops.rmsnorm_quant(x[r:r + 1, :h], w, 1e-6, res[r:r + 1, :h], gemma=True)
         assert torch.equal(q1.view(torch.uint8)[0], xq[r]) and torch.equal(s1[0], sx[:, r])
-    rows = torch.tensor([0, 149, m - 1])
+    rows = torch.tensor([0, sm + 1, m - 1])
     ref, _ = R.rms_norm(x[rows.cuda(), :h].cpu(), w.cpu(), 1e-6, res[rows.cuda(), :h].cpu(), gemma=True)
     if h > 16:                                              # 48 bytes are too few for a share of equal ones
         check_quantised(xq[rows.cuda()].view(torch.float8_e4m3fn), sx[:, rows.cuda()].t(), ref)
@@ -194,13 +195,15 @@ def test_rmsnorm_quant_order_of_the_sum(ops, h, m):
     assert torch.equal(y[-3:].view(torch.int16), want.view(torch.int16))
 
 
-@pytest.mark.parametrize("m", [1, 888, 889])
-def test_silu_mul_quant_narrow_and_wide_lanes(ops, m):
-    """Groups of 8 elements per lane up to one wave of CTAs (148 SMs: 14208 groups = 888 rows of 16), of 16 beyond: the same
+@pytest.mark.parametrize("beyond", [None, 0, 1])
+def test_silu_mul_quant_narrow_and_wide_lanes(ops, beyond):
+    """Groups of 8 elements per lane up to one wave of CTAs (96 groups per SM: 6 rows of 16), of 16 beyond: the same
     bytes either side, rows that end inside a group, and the values the arithmetic has to carry through."""
     inter = 16 * 128 - 112
+    wave = 6 * torch.cuda.get_device_properties(0).multi_processor_count
+    m = 1 if beyond is None else wave + beyond
     gen = torch.Generator().manual_seed(5)
-    gu = (torch.randn(889, 2 * inter, generator=gen) * 4.0).to(torch.bfloat16)
+    gu = (torch.randn(wave + 1, 2 * inter, generator=gen) * 4.0).to(torch.bfloat16)
     gu[0, :4] = torch.tensor([-0.0, 90.0, -90.0, 1e-30])
     gu[0, inter:inter + 4] = torch.tensor([1.0, -0.0, 3.0, 2.0])
     xq, sx = ops.silu_mul_quant(gu[:m].cuda())
